@@ -201,7 +201,9 @@ typedef struct {
     void *geo;              /* FP32C float4[N]: 2D {xr,yr,h,m}, 3D {xr,yr,zr,h} */
     void *mass;             /* FP32C 3D float[N]: m */
     void *vel;              /* FP32C: 2D float2 {u,v}, 3D float4 {u,v,w,0} */
-    void *thermo;           /* FP32C float4[N]: {rho, p, cs, p/rho^2} */
+    void *thermo;           /* FP32C float4[N]: {rho, p, cs, p/rho^2};
+                               FP64 double[N]: p/rho^2 (may be NULL: the
+                               force pass then takes it per pair) */
     int32_t *cell;          /* local cell index of each particle */
     /* Neighbour lists of the last sphb_density pass (optional, may be
      * NULL): uint32 [list_cap][N] slot-major, entry = j | cell offsets

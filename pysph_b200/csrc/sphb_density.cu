@@ -56,6 +56,7 @@ k_tait(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask)
         if (state) ((double *)e.f.rho)[k] = rho;
         ((double *)e.f.p)[k] = p;
         ((double *)e.f.cs)[k] = c;
+        if (e.f.thermo) ((double *)e.f.thermo)[k] = p * (1.0 / (rho * rho));
         if (state && !(isfinite(rho) && isfinite(p))) flag(e, SPHB_ST_NONFINITE_RHO);
     }
 }

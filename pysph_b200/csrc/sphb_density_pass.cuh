@@ -67,6 +67,9 @@ __device__ __forceinline__ void density_finish(const sphb_engine &e, int cur, in
                 ((double *)e.f.p)[k] = p;
                 ((double *)e.f.cs)[k] = c;
             }
+            // the force pass's P / rho^2, once per particle instead of per pair
+            if (e.f.thermo && e.f.p)
+                ((double *)e.f.thermo)[k] = (eos ? p : ((double *)e.f.p)[k]) * (1.0 / (rho * rho));
             if (!isfinite(rho) || !isfinite(p)) flag(e, SPHB_ST_NONFINITE_RHO);
         }
     }
@@ -205,7 +208,7 @@ k_density(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask, in
                         const float rj = hj * rsf;   // r < radius_scale max(h_a, h_b)
                         if (!(r2 < rad2 || r2 < rj * rj)) return;
                     }
-                    const float ir = rsqrtf(fmaxf(r2, 1e-30f));   // q = 0 at r = 0
+                    const float ir = inv_dist(r2);   // q = 0 at r = 0
                     float w;
                     if (UH) {
                         w = Kern<KT>::w_bf(r2 * ir * ihk, fack);
@@ -245,7 +248,7 @@ k_density(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask, in
                 };
                 auto sum_plain = [&](const Rec &r, float r2) {
                     if (r2 < rad2) {
-                        const float ir = rsqrtf(fmaxf(r2, 1e-30f));   // q = 0 at r = 0
+                        const float ir = inv_dist(r2);   // q = 0 at r = 0
                         acc.add(r.m * Kern<KT>::w_bf(r2 * ir * ihk, fack));
                         ++np;
                     }
@@ -253,12 +256,16 @@ k_density(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask, in
                 const int lc = list_count<LANES>(e, from_list, k, lane);
                 if (lc >= 0) {
                     if (plain) {
-                        list_loop<DIM, LANES, 4>(e, k, lane, lc, load_all,
-                                                 [&](const Rec &r) { sum_plain(r, dist2(r)); });
+                        list_loop<LANES, 4>(
+                            e, k, lane, lc,
+                            [&](uint32_t v) { return load_all(entry_unpack_f<DIM>(v)); },
+                            [&](const Rec &r) { sum_plain(r, dist2(r)); });
                         return;
                     }
-                    list_loop<DIM, LANES, 4>(e, k, lane, lc, load,
-                                             [&](const Rec &r) { use(r, dist2(r)); });
+                    list_loop<LANES, 4>(
+                        e, k, lane, lc,
+                        [&](uint32_t v) { return load(entry_unpack_f<DIM>(v)); },
+                        [&](const Rec &r) { use(r, dist2(r)); });
                     return;
                 }
                 int cx, cy, cz;
@@ -316,45 +323,92 @@ k_density(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask, in
             const double rad2 = __dmul_rn(rad, rad);
             const double radl = (rad + skin) * (1.0 + 1e-5);
             const double radl2 = nbr ? radl * radl : rad2;
+            const double kf = Kern<KT>::template norm<DIM>();
+            const double ihk = 1.0 / hk;
+            const double fack = DIM == 2 ? kf * ihk * ihk : kf * ihk * ihk * ihk;
             // with one h in the scene the symmetric set and the averaged
             // kernel are the plain ones
-            const bool uh = sc.uniform_h != 0;
-            const bool vh = !uh && sc.variable_h != 0, hks = !uh && sc.hks != 0;
-            int cx, cy, cz;
-            cell_coords(e.f.cell[k], n, cx, cy, cz);
-            traverse<DIM, R, LANES>(
-                e, from_list, k, lane, start, A, src, cell_base, ncells, n, cx, cy, cz,
-                cell_trim_abs<DIM>(e, st, sc.cell_size, xk, yk, zk, cx, cy, cz),
-                [&](int j, int o, int oy, int oz) {
-                    const double dx = xk - __ldg(B.x + j);
-                    const double dy = yk - __ldg(B.y + j);
-                    const double dz = DIM == 3 ? zk - __ldg(B.z + j) : 0.0;
-                    const double d2 = dist2_ref<DIM>(dx, dy, dz);
-                    double hb = 0.0, radj2 = rad2, radlj2 = radl2;
-                    if (vh) {
-                        // symmetric: r^2 < (radius_scale h_a)^2 or (radius_scale h_b)^2
-                        hb = __ldg(B.h + j);
-                        const double rj = hb * sc.radius_scale;
+            const bool vh = sc.variable_h != 0, hks = sc.hks != 0;
+            struct Rec {
+                double x, y, z, m, h;
+                bool ok;
+            };
+            auto pass = [&](auto uniform) {
+                constexpr bool UH = decltype(uniform)::value;
+                auto load = [&](int j, bool ok) {
+                    Rec r;
+                    r.ok = ok && (!filt || ((rsrc >> seg.array_of(j)) & 1u));
+                    r.x = __ldg(B.x + j);
+                    r.y = __ldg(B.y + j);
+                    r.z = DIM == 3 ? __ldg(B.z + j) : 0.0;
+                    r.m = __ldg(B.m + j);
+                    r.h = UH ? hk : __ldg(B.h + j);
+                    return r;
+                };
+                auto dist2 = [&](const Rec &r) {
+                    return dist2_ref<DIM>(xk - r.x, yk - r.y, DIM == 3 ? zk - r.z : 0.0);
+                };
+                auto use = [&](const Rec &r, double d2) {
+                    // symmetric: r^2 < (radius_scale h_a)^2 or (radius_scale h_b)^2
+                    double radj2 = rad2;
+                    if (!UH && vh) {
+                        const double rj = r.h * sc.radius_scale;
                         radj2 = fmax(rad2, __dmul_rn(rj, rj));
-                        const double rl = (fmax(rad, rj) + skin) * (1.0 + 1e-5);
-                        radlj2 = nbr ? rl * rl : radj2;
                     }
-                    if (d2 < radlj2) {
-                        record(j, o, oy, oz);
-                        const bool sums =
-                            !lists_only && (!filt || ((rsrc >> seg.array_of(j)) & 1u));
-                        if (sums && d2 < radj2) {
-                            if (!vh) hb = uh ? hk : __ldg(B.h + j);
-                            double w;
-                            if (hks)
-                                w = 0.5 * (Kern<KT>::template w_d<DIM>(sqrt(d2), hk) + Kern<KT>::template w_d<DIM>(sqrt(d2), hb));
-                            else
-                                w = Kern<KT>::template w_d<DIM>(sqrt(d2), 0.5 * (hk + hb));
-                            sum += w * __ldg(B.m + j);
-                            ++np;
+                    if (!r.ok || !(d2 < radj2)) return;
+                    const double ir = inv_dist(d2);
+                    double w;
+                    if (UH) {
+                        w = Kern<KT>::w_bf(d2 * ir * ihk, fack);
+                    } else {
+                        // W(r, h_ab), or with hks (W(r, h_a) + W(r, h_b)) / 2
+                        const double rr = d2 * ir;
+                        double hs = hks ? hk : 0.5 * (hk + r.h);
+                        w = 0.0;
+#pragma unroll 1
+                        for (int t = 0;; ++t) {
+                            const double ih = 1.0 / hs;
+                            w += Kern<KT>::w_bf(rr * ih,
+                                                DIM == 2 ? kf * ih * ih : kf * ih * ih * ih);
+                            if (!hks || t == 1) break;
+                            hs = r.h;
                         }
+                        if (hks) w *= 0.5;
                     }
-                });
+                    sum += r.m * w;
+                    ++np;
+                };
+                const int lc = list_count<LANES>(e, from_list, k, lane);
+                if (lc >= 0) {
+                    list_loop<LANES, 4>(
+                        e, k, lane, lc,
+                        [&](uint32_t v) {
+                            int j;
+                            const bool ok = list_entry_d<DIM>(e, v, k, j);
+                            return load(j, ok);
+                        },
+                        [&](const Rec &r) { use(r, dist2(r)); });
+                    return;
+                }
+                int cx, cy, cz;
+                cell_coords(e.f.cell[k], n, cx, cy, cz);
+                for_each_candidate<DIM, R, LANES>(
+                    start, A, src, cell_base, ncells, n, cx, cy, cz, lane, N, e.work.status,
+                    cell_trim_abs<DIM>(e, st, sc.cell_size, xk, yk, zk, cx, cy, cz),
+                    [&](int j, int o, int oy, int oz) {
+                        const Rec r = load(j, !lists_only);
+                        const double d2 = dist2(r);
+                        bool rec = d2 < radl2;
+                        if (!UH && vh && nbr && !rec) {
+                            const double rl = (r.h * sc.radius_scale + skin) * (1.0 + 1e-5);
+                            rec = r.h > hk && d2 < rl * rl;
+                        }
+                        if (rec) record(j, o, oy, oz);
+                        use(r, d2);
+                    });
+            };
+            if (sc.uniform_h) pass(std::true_type{});
+            else pass(std::false_type{});
         }
 #pragma unroll
         for (int o = LANES / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);

@@ -131,6 +131,16 @@ __device__ __forceinline__ void force_finish(const sphb_engine &e, int cur, int 
     block_add_u64(&e.work.pairs[1], np);
 }
 
+// List entries the FP64 force pass loads ahead.  The FP64 pair was bound by
+// its own latency: one neighbour at a time, four dependent rounds of loads
+// (position; h, rho, p, m; velocity; cs) and eight divisions and a square
+// root in branches.  With every field of a batch loaded up front, P / rho^2
+// kept per particle, one reciprocal square root and the dest's 1 / h instead
+// of the kernel's divisions, the pass with the density pass it overlaps goes
+// 134 -> 63 us on an 86k-particle 2D dam break and 95 -> 40 us on a 5k drop
+// (one lane per particle); batches of 4 do not fit 128 registers.
+constexpr int FP64_BATCH = 2;
+
 // CONT: the continuity scheme's pair terms too -- SPHDensityRate
 // (density_funcs.pyx:119-156) and XSPHCorrection (xsph_funcs.pyx:40-86),
 // each over its own sources, in the same traversal as the momentum.
@@ -300,7 +310,7 @@ k_force(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask,
                         float dot = vx * rx + vy * ry;
                         if (DIM == 3) dot += vz * rz;
                         // r = 0 (self) gives q = 0 and a finite gradient times r_ab = 0
-                        const float ir = rsqrtf(fmaxf(r2, 1e-30f));
+                        const float ir = inv_dist(r2);
                         // grad W / r (and W for XSPH) at h_ab, or with hks the means
                         // of the values at h_a and h_b: one evaluation in a loop
                         // keeps the register count of the uniform-h path
@@ -360,20 +370,21 @@ k_force(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask,
                         if (DIM == 3) az.add(f * rz);
                     };
                 };
+                auto load_entry = [&](uint32_t v) { return load(entry_unpack_f<DIM>(v)); };
                 const int lc = list_count<LANES>(e, use_list, k, lane);
                 if (lc >= 0) {
                     switch (mode & 15) {   // block-uniform
                     case 0:
-                        list_loop<DIM, LANES, U>(e, k, lane, lc, load,
-                                                 make_use(std::integral_constant<int, 0>{}));
+                        list_loop<LANES, U>(e, k, lane, lc, load_entry,
+                                            make_use(std::integral_constant<int, 0>{}));
                         break;
                     case 1:
-                        list_loop<DIM, LANES, U>(e, k, lane, lc, load,
-                                                 make_use(std::integral_constant<int, 1>{}));
+                        list_loop<LANES, U>(e, k, lane, lc, load_entry,
+                                            make_use(std::integral_constant<int, 1>{}));
                         break;
                     default:
-                        list_loop<DIM, LANES, U>(e, k, lane, lc, load,
-                                                 make_use(std::integral_constant<int, 2>{}));
+                        list_loop<LANES, U>(e, k, lane, lc, load_entry,
+                                            make_use(std::integral_constant<int, 2>{}));
                         break;
                     }
                     return;
@@ -419,110 +430,185 @@ k_force(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask,
         }
     } else {
         if (active) {
+            const int N = e.cfg.num_particles;
             const sphb_buffers &B = e.buf[cur];
             const double *__restrict__ rho = (const double *)e.f.rho;
             const double *__restrict__ pr = (const double *)e.f.p;
             const double *__restrict__ csnd = (const double *)e.f.cs;
+            // P / rho^2 as the density pass and the Tait kernel left it; a
+            // caller without the field has it taken per pair
+            const double *__restrict__ prho2 = (const double *)e.f.thermo;
             const double xk = B.x[k], yk = B.y[k], zk = DIM == 3 ? B.z[k] : 0.0;
             const double uk = B.u[k], vk = B.v[k], wk = DIM == 3 ? B.w[k] : 0.0;
             const double hk = B.h[k];
-            const double rhoa = rho[k], Pa = pr[k], ca = csnd[k];
-            const double rhoa2 = 1.0 / (rhoa * rhoa);
+            const double rhoa = rho[k], ca = csnd[k];
+            auto p_rho2 = [&](int j) {
+                if (prho2) return __ldg(prho2 + j);
+                const double r = __ldg(rho + j);
+                return __ldg(pr + j) * (1.0 / (r * r));
+            };
+            const double ta = p_rho2(k);
             const double rad = hk * sc.radius_scale;
             const double rad2 = __dmul_rn(rad, rad);
-            const double alpha = sc.alpha, beta = sc.beta, eta = sc.eta;
+            const double alpha = sc.alpha, beta = sc.beta, eta2 = sc.eta * sc.eta;
+            const double kf = Kern<KT>::template norm<DIM>();
+            const double ihk = 1.0 / hk;
+            const double fihk = DIM == 2 ? kf * ihk * ihk * ihk : kf * ihk * ihk * ihk * ihk;
             // with one h in the scene the symmetric set and the averaged
             // kernels are the plain ones
-            const bool uh = sc.uniform_h != 0;
-            const bool vh = !uh && sc.variable_h != 0, hks = !uh && sc.hks != 0;
-            int cx, cy, cz;
-            cell_coords(e.f.cell[k], n, cx, cy, cz);
-            traverse<DIM, R, LANES>(
-                e, use_list, k, lane, start, A, src, cell_base, ncells, n, cx, cy, cz,
-                cell_trim_abs<DIM>(e, st, sc.cell_size, xk, yk, zk, cx, cy, cz),
-                [&](int j, int, int, int) {
-                    const double rx = xk - __ldg(B.x + j);
-                    const double ry = yk - __ldg(B.y + j);
-                    const double rz = DIM == 3 ? zk - __ldg(B.z + j) : 0.0;
-                    const double rab2 = dist2_ref<DIM>(rx, ry, rz);
-                    double hb = 0.0, radj2 = rad2;
-                    if (vh) {
-                        // symmetric: r^2 < (radius_scale h_a)^2 or (radius_scale h_b)^2
-                        hb = __ldg(B.h + j);
-                        const double rj = hb * sc.radius_scale;
-                        radj2 = fmax(rad2, __dmul_rn(rj, rj));
-                    }
-                    if (!(rab2 < radj2)) return;
-                    if (!vh) hb = uh ? hk : __ldg(B.h + j);
-                    ++np;
-                    const uint32_t bit = filt ? 1u << seg.array_of(j) : ~0u;
-                    const double hab = 0.5 * (hk + hb);
-                    const double rhob = __ldg(rho + j), Pb = __ldg(pr + j);
-                    const double mb = __ldg(B.m + j);
-                    // grad_a W: at h_ab, or with hks the mean of the gradients
-                    // at h_a and h_b (pressure_funcs.pyx:371-381)
-                    double gx, gy, gz = 0.0;
-                    if (hks) {
-                        const double ga = Kern<KT>::template gw_d<DIM>(sqrt(rab2), hk);
-                        const double gb = Kern<KT>::template gw_d<DIM>(sqrt(rab2), hb);
-                        gx = (rx * ga + rx * gb) * 0.5;
-                        gy = (ry * ga + ry * gb) * 0.5;
-                        if (DIM == 3) gz = (rz * ga + rz * gb) * 0.5;
-                    } else {
-                        const double g = Kern<KT>::template gw_d<DIM>(sqrt(rab2), hab);
-                        gx = rx * g;
-                        gy = ry * g;
-                        if (DIM == 3) gz = rz * g;
-                    }
-                    if (CONT) {
-                        const double vbx = __ldg(B.u + j), vby = __ldg(B.v + j);
-                        const double vbz = DIM == 3 ? __ldg(B.w + j) : 0.0;
-                        if (rm & bit) {
-                            // SPHDensityRate: ((v_a - v_b) . grad_a W) m_b
-                            double d = (uk - vbx) * gx + (vk - vby) * gy;
-                            if (DIM == 3) d += (wk - vbz) * gz;
-                            drho += d * mb;
+            const bool vh = sc.variable_h != 0, hks = sc.hks != 0;
+            struct Rec {
+                double x, y, z, u, v, w, m, h, rho, t, c;
+                uint32_t bit;   // the source's array as a mask bit (CONT)
+                bool ok;
+            };
+            auto pass = [&](auto uniform) {
+                constexpr bool UH = decltype(uniform)::value;
+                // KM as in the FP32C body: the mode known at compile time in
+                // the list loops, -1 in the cell search
+                auto make_load = [&](auto known) {
+                    constexpr int KM = decltype(known)::value;
+                    return [&](int j, bool ok) {
+                        Rec r;
+                        r.ok = ok;
+                        r.bit = filt ? 1u << seg.array_of(j) : ~0u;
+                        r.x = __ldg(B.x + j);
+                        r.y = __ldg(B.y + j);
+                        r.z = DIM == 3 ? __ldg(B.z + j) : 0.0;
+                        r.m = __ldg(B.m + j);
+                        r.h = UH ? hk : __ldg(B.h + j);
+                        r.t = KM == 2 ? 0.0 : p_rho2(j);
+                        r.u = r.v = r.w = r.rho = r.c = 0.0;
+                        if (KM != 1 || CONT) {
+                            r.u = __ldg(B.u + j);
+                            r.v = __ldg(B.v + j);
+                            if (DIM == 3) r.w = __ldg(B.w + j);
+                            r.rho = __ldg(rho + j);
                         }
-                        if (xm & bit) {
-                            // XSPHCorrection: m_b W_ab / rho_ab (v_b - v_a) eps
-                            const double w =
-                                hks ? 0.5 * (Kern<KT>::template w_d<DIM>(sqrt(rab2), hk) +
-                                             Kern<KT>::template w_d<DIM>(sqrt(rab2), hb))
-                                    : Kern<KT>::template w_d<DIM>(sqrt(rab2), hab);
-                            const double temp = mb * w / (0.5 * (rhob + rhoa));
-                            xs[0] += temp * (vbx - uk) * sc.xsph_eps;
-                            xs[1] += temp * (vby - vk) * sc.xsph_eps;
-                            if (DIM == 3) xs[2] += temp * (vbz - wk) * sc.xsph_eps;
+                        if (KM != 1) r.c = __ldg(csnd + j);
+                        return r;
+                    };
+                };
+                auto make_use = [&](auto known) {
+                    constexpr int KM = decltype(known)::value;
+                    const bool visc_k = KM < 0 ? visc : KM == 0;
+                    const bool avisc_k = KM < 0 ? avisc : KM == 2;
+                    return [&, visc_k, avisc_k](const Rec &r) {
+                        const double rx = xk - r.x, ry = yk - r.y;
+                        const double rz = DIM == 3 ? zk - r.z : 0.0;
+                        const double r2 = dist2_ref<DIM>(rx, ry, rz);
+                        double radj2 = rad2;
+                        if (!UH && vh) {
+                            // symmetric: r^2 < (radius_scale h_a)^2 or (radius_scale h_b)^2
+                            const double rj = r.h * sc.radius_scale;
+                            radj2 = fmax(rad2, __dmul_rn(rj, rj));
                         }
-                        if (!(mm & bit)) return;
-                    }
-                    // P_a/rho_a^2 + P_b/rho_b^2; the split viscosity has none
-                    // (tmp = piab; tmp *= -mb, viscosity_funcs.pyx:125-126)
-                    double tmp = avisc ? 0.0 : Pa * rhoa2 + Pb * (1.0 / (rhob * rhob));
-                    if (visc || avisc) {
-                        const double vx = uk - __ldg(B.u + j);
-                        const double vy = vk - __ldg(B.v + j);
-                        const double vz = DIM == 3 ? wk - __ldg(B.w + j) : 0.0;
-                        double dot = vx * rx + vy * ry;
-                        if (DIM == 3) dot += vz * rz;
-                        const double den = rab2 + eta * eta * hab * hab;
-                        dtf = fmax(dtf, fabs(hab * dot /
-                                             (avisc ? rab2 + 0.01 * hab * hab : den)));
-                        if (dot < 0) {
-                            const double cab = 0.5 * (ca + __ldg(csnd + j));
-                            const double rhoab = 0.5 * (rhoa + rhob);
-                            double mu = hab * dot;
-                            mu /= den;
-                            double piab = -alpha * cab * mu + beta * mu * mu;
-                            piab /= rhoab;
-                            tmp += piab;
+                        if (!r.ok || !(r2 < radj2)) return;
+                        ++np;
+                        const bool mom_on = !CONT || (mm & r.bit);
+                        const bool rate_on = CONT && (rm & r.bit);
+                        const bool xs_on = CONT && (xm & r.bit);
+                        const double hab = UH ? hk : 0.5 * (hk + r.h);
+                        const double ir = inv_dist(r2);
+                        // grad W / r (and W for XSPH) at h_ab, or with hks the
+                        // means of the values at h_a and h_b (pressure_funcs.pyx:
+                        // 371-381)
+                        double gw, w = 0.0;
+                        if (UH) {
+                            const double q = r2 * ir * ihk;
+                            gw = Kern<KT>::gw_bf(q, ir, ihk, fihk);
+                            if (CONT && xs_on) w = Kern<KT>::w_bf(q, fihk * hk);
+                        } else {
+                            const double rr = r2 * ir;
+                            double hs = hks ? hk : hab;
+                            gw = 0.0;
+#pragma unroll 1
+                            for (int t = 0;; ++t) {
+                                const double ih = 1.0 / hs;
+                                const double fih = DIM == 2 ? kf * ih * ih * ih
+                                                            : kf * ih * ih * ih * ih;
+                                const double q = rr * ih;
+                                gw += Kern<KT>::gw_bf(q, ir, ih, fih);
+                                if (CONT && xs_on) w += Kern<KT>::w_bf(q, fih * hs);
+                                if (!hks || t == 1) break;
+                                hs = r.h;
+                            }
+                            if (hks) {
+                                gw *= 0.5;
+                                w *= 0.5;
+                            }
                         }
+                        const double gx = rx * gw, gy = ry * gw, gz = rz * gw;
+                        const double vx = uk - r.u, vy = vk - r.v, vz = wk - r.w;
+                        if (CONT) {
+                            if (rate_on) {
+                                // SPHDensityRate: ((v_a - v_b) . grad_a W) m_b
+                                double d = vx * gx + vy * gy;
+                                if (DIM == 3) d += vz * gz;
+                                drho += d * r.m;
+                            }
+                            if (xs_on) {
+                                // XSPHCorrection: m_b W_ab / rho_ab (v_b - v_a) eps
+                                const double temp =
+                                    r.m * w / (0.5 * (r.rho + rhoa)) * sc.xsph_eps;
+                                xs[0] -= temp * vx;
+                                xs[1] -= temp * vy;
+                                if (DIM == 3) xs[2] -= temp * vz;
+                            }
+                            if (!mom_on) return;
+                        }
+                        // P_a/rho_a^2 + P_b/rho_b^2; the split viscosity has none
+                        // (tmp = piab; tmp *= -mb, viscosity_funcs.pyx:125-126)
+                        double tmp = avisc_k ? 0.0 : ta + r.t;
+                        if (visc_k || avisc_k) {
+                            double dot = vx * rx + vy * ry;
+                            if (DIM == 3) dot += vz * rz;
+                            const double hd = hab * dot;
+                            const double mu = hd / (r2 + eta2 * hab * hab);
+                            dtf = fmax(dtf, fabs(avisc_k ? hd / (r2 + 0.01 * hab * hab) : mu));
+                            // Monaghan Pi_ab when v_ab . r_ab < 0, selected, not branched on
+                            const double cab = 0.5 * (ca + r.c);
+                            const double rhoab = 0.5 * (rhoa + r.rho);
+                            const double piab = (-alpha * cab * mu + beta * mu * mu) / rhoab;
+                            tmp += dot < 0.0 ? piab : 0.0;
+                        }
+                        tmp *= -r.m;
+                        acc[0] += tmp * gx;
+                        acc[1] += tmp * gy;
+                        if (DIM == 3) acc[2] += tmp * gz;
+                    };
+                };
+                const int lc = list_count<LANES>(e, use_list, k, lane);
+                if (lc >= 0) {
+                    auto from_list = [&](auto known) {
+                        auto load = make_load(known);
+                        list_loop<LANES, FP64_BATCH>(
+                            e, k, lane, lc,
+                            [&](uint32_t v) {
+                                int j;
+                                const bool ok = list_entry_d<DIM>(e, v, k, j);
+                                return load(j, ok);
+                            },
+                            make_use(known));
+                    };
+                    switch (mode & 15) {   // block-uniform
+                    case 0: from_list(std::integral_constant<int, 0>{}); break;
+                    case 1: from_list(std::integral_constant<int, 1>{}); break;
+                    default: from_list(std::integral_constant<int, 2>{}); break;
                     }
-                    tmp *= -mb;
-                    acc[0] += tmp * gx;
-                    acc[1] += tmp * gy;
-                    if (DIM == 3) acc[2] += tmp * gz;
-                });
+                    return;
+                }
+                auto load = make_load(std::integral_constant<int, -1>{});
+                auto use = make_use(std::integral_constant<int, -1>{});
+                int cx, cy, cz;
+                cell_coords(e.f.cell[k], n, cx, cy, cz);
+                for_each_candidate<DIM, R, LANES>(
+                    start, A, src, cell_base, ncells, n, cx, cy, cz, lane, N, e.work.status,
+                    cell_trim_abs<DIM>(e, st, sc.cell_size, xk, yk, zk, cx, cy, cz),
+                    [&](int j, int, int, int) { use(load(j, true)); });
+            };
+            if (sc.uniform_h) pass(std::true_type{});
+            else pass(std::false_type{});
         }
 #pragma unroll
         for (int o = LANES / 2; o > 0; o >>= 1) {

@@ -2,21 +2,25 @@
 //
 // Kern<KT> (KT = SPHB_KERNEL_*) gives, for one kernel type:
 //   norm<DIM>()             _fac(1.0), the normalisation at h = 1
-//   w_bf(q, fac)            W = fac val(q), FP32, branch-free (every piece
+//   w_bf(q, fac)            W = fac val(q), branch-free (every piece
 //                           computed, one selected) for the list loops
 //   gw_bf(q, ir, ih, fac_ih) dW/dr / r in the reference's sign convention,
-//                           so grad_a W = (x_a - x_b) gw; FP32
-//   w_d<DIM>(r, h), gw_d<DIM>(r, h)  the FP64 forms with the reference's
-//                           operations in its order
-// with fac = norm<DIM>() / h^DIM, ih = 1 / h, ir = 1 / r, fac_ih = fac ih.
-// For r = 0 the FP32 forms see ir = 1/sqrt(1e-30) (finite); every caller
-// multiplies gw by r_ab = 0 there.
+//                           so grad_a W = (x_a - x_b) gw
+// with fac = norm<DIM>() / h^DIM, ih = 1 / h, ir = 1 / r, fac_ih = fac ih,
+// for T = float and double.  No form divides: the pair loops take one
+// reciprocal square root per pair and, with one h in the scene, the dest's
+// 1 / h.  For r = 0 they see a finite ir (inv_dist); every caller multiplies
+// gw by r_ab = 0 there.
 
 #pragma once
 
 #include "sphb_common.cuh"
 
 namespace sphb {
+
+// 1 / r from r^2; finite at r = 0, where r^2 times it is 0.
+__device__ __forceinline__ float inv_dist(float r2) { return rsqrtf(fmaxf(r2, 1e-30f)); }
+__device__ __forceinline__ double inv_dist(double r2) { return rsqrt(fmax(r2, 1e-200)); }
 
 template <int KT>
 struct Kern;
@@ -29,51 +33,23 @@ struct Kern<SPHB_KERNEL_CUBIC> {
     __host__ __device__ static double norm() { return kfac_unit<DIM>(); }
 
     // q < 1: 1 + q^2 (0.75 q - 1.5); else t1^3 / 4 with t1 = max(2 - q, 0)
-    __device__ __forceinline__ static float w_bf(float q, float fac)
+    template <typename T>
+    __device__ __forceinline__ static T w_bf(T q, T fac)
     {
-        const float t1 = fmaxf(2.0f - q, 0.0f);
-        const float inner = fmaf(q * q, fmaf(0.75f, q, -1.5f), 1.0f);
-        const float outer = 0.25f * (t1 * t1 * t1);
-        return fac * (q < 1.0f ? inner : outer);
+        const T t1 = fmax(T(2) - q, T(0));
+        const T inner = fma(q * q, fma(T(0.75), q, T(-1.5)), T(1));
+        const T outer = T(0.25) * (t1 * t1 * t1);
+        return fac * (q < T(1) ? inner : outer);
     }
 
     // q < 1: (2.25 q - 3) ih; else -0.75 t1^2 / r
-    __device__ __forceinline__ static float gw_bf(float q, float ir, float ih, float fac_ih)
+    template <typename T>
+    __device__ __forceinline__ static T gw_bf(T q, T ir, T ih, T fac_ih)
     {
-        const float t1 = fmaxf(2.0f - q, 0.0f);
-        const float inner = (2.25f * q - 3.0f) * ih;
-        const float outer = -0.75f * t1 * t1 * ir;
-        return fac_ih * (q < 1.0f ? inner : outer);
-    }
-
-    template <int DIM>
-    __device__ __forceinline__ static double w_d(double rab, double h)
-    {
-        const double q = rab / h;
-        double val;
-        const double fac = (DIM == 2 ? 1.0 / (h * h) : 1.0 / (h * h * h)) * kfac_unit<DIM>();
-        if (q > 2.0)
-            val = 0.0;
-        else if (q > 1.0)
-            val = 0.25 * (2 - q) * (2 - q) * (2 - q);
-        else
-            val = 1 - 1.5 * (q * q) * (1 - 0.5 * q);
-        return val * fac;
-    }
-
-    template <int DIM>
-    __device__ __forceinline__ static double gw_d(double rab, double h)
-    {
-        const double q = rab / h;
-        double val = 0.0;
-        const double fac = (DIM == 2 ? 1.0 / (h * h) : 1.0 / (h * h * h)) * kfac_unit<DIM>();
-        if (q > 2.0) {
-        } else if (q >= 1.0) {
-            val = -0.75 * (2 - q) * (2 - q) / (h * rab);
-        } else if (q > 1e-14) {
-            val = 3.0 * (0.75 * q - 1) / (h * h);
-        }
-        return val * fac;
+        const T t1 = fmax(T(2) - q, T(0));
+        const T inner = (T(2.25) * q - T(3)) * ih;
+        const T outer = T(-0.75) * t1 * t1 * ir;
+        return fac_ih * (q < T(1) ? inner : outer);
     }
 };
 
@@ -89,81 +65,29 @@ struct Kern<SPHB_KERNEL_QUINTIC> {
         return DIM == 2 ? 7. / (478 * 3.141592653589793 * 1.0 * 1.0) : 0.0;
     }
 
-    __device__ __forceinline__ static float p4(float t)
+    template <typename T>
+    __device__ __forceinline__ static T p4(T t)
     {
-        const float t2 = t * t;
+        const T t2 = t * t;
         return t2 * t2;
     }
 
-    __device__ __forceinline__ static float w_bf(float q, float fac)
+    template <typename T>
+    __device__ __forceinline__ static T w_bf(T q, T fac)
     {
-        const float t3 = fmaxf(3.0f - q, 0.0f);
-        const float t2 = fmaxf(2.0f - q, 0.0f);
-        const float t1 = fmaxf(1.0f - q, 0.0f);
-        return fac * fmaf(p4(t1), t1, fmaf(-6.0f * p4(t2), t2, p4(t3) * t3));
+        const T t3 = fmax(T(3) - q, T(0));
+        const T t2 = fmax(T(2) - q, T(0));
+        const T t1 = fmax(T(1) - q, T(0));
+        return fac * fma(p4(t1), t1, fma(T(-6) * p4(t2), t2, p4(t3) * t3));
     }
 
-    __device__ __forceinline__ static float gw_bf(float q, float ir, float, float fac_ih)
+    template <typename T>
+    __device__ __forceinline__ static T gw_bf(T q, T ir, T, T fac_ih)
     {
-        const float t3 = fmaxf(3.0f - q, 0.0f);
-        const float t2 = fmaxf(2.0f - q, 0.0f);
-        const float t1 = fmaxf(1.0f - q, 0.0f);
-        return fac_ih * ir * fmaf(75.0f, p4(t1), fmaf(-30.0f, p4(t2), 5.0f * p4(t3)));
-    }
-
-    template <int DIM>
-    __device__ __forceinline__ static double w_d(double rab, double h)
-    {
-        const double fac = norm<DIM>() * (1.0 / (h * h));
-        const double q = rab / h;
-        double val;
-        double tmp1 = (3 - q), tmp2 = (2 - q), tmp3 = (1 - q);
-        if (q > 3.0) {
-            val = 0.0;
-        } else {
-            tmp1 = __dmul_rn(tmp1, __dmul_rn(__dmul_rn(__dmul_rn(tmp1, tmp1), tmp1), tmp1));
-            if (q > 2.0) {
-                val = tmp1;
-            } else {
-                tmp2 = __dmul_rn(tmp2, __dmul_rn(__dmul_rn(__dmul_rn(tmp2, tmp2), tmp2), tmp2));
-                val = __dsub_rn(tmp1, __dmul_rn(6.0, tmp2));
-                if (!(q > 1.0)) {
-                    tmp3 = __dmul_rn(tmp3, __dmul_rn(__dmul_rn(__dmul_rn(tmp3, tmp3), tmp3), tmp3));
-                    val = __dadd_rn(val, tmp3);
-                }
-            }
-        }
-        return val * fac;
-    }
-
-    template <int DIM>
-    __device__ __forceinline__ static double gw_d(double rab, double h)
-    {
-        double fac = norm<DIM>() * (1.0 / (h * h));
-        const double q = rab / h;
-        double val;
-        double tmp1 = (3 - q), tmp2 = (2 - q), tmp3 = (1 - q);
-        if (rab < 1e-16) {
-            val = 0.0;
-        } else {
-            fac *= 1. / (h * rab);
-            if (q > 3.0) {
-                val = 0.0;
-            } else {
-                tmp1 = __dmul_rn(tmp1, __dmul_rn(__dmul_rn(tmp1, tmp1), tmp1));
-                if (q > 2.0) {
-                    val = __dmul_rn(5.0, tmp1);
-                } else {
-                    tmp2 = __dmul_rn(tmp2, __dmul_rn(__dmul_rn(tmp2, tmp2), tmp2));
-                    val = __dsub_rn(__dmul_rn(5.0, tmp1), __dmul_rn(30.0, tmp2));
-                    if (!(q > 1.0)) {
-                        tmp3 = __dmul_rn(tmp3, __dmul_rn(__dmul_rn(tmp3, tmp3), tmp3));
-                        val = __dadd_rn(val, __dmul_rn(75.0, tmp3));
-                    }
-                }
-            }
-        }
-        return val * fac;
+        const T t3 = fmax(T(3) - q, T(0));
+        const T t2 = fmax(T(2) - q, T(0));
+        const T t1 = fmax(T(1) - q, T(0));
+        return fac_ih * ir * fma(T(75), p4(t1), fma(T(-30), p4(t2), T(5) * p4(t3)));
     }
 };
 
@@ -178,56 +102,20 @@ struct Kern<SPHB_KERNEL_WENDLAND> {
         return DIM == 2 ? (7. / 4 * 3.141592653589793 * 1.0 * 1.0) : 0.0;
     }
 
-    __device__ __forceinline__ static float w_bf(float q, float fac)
+    template <typename T>
+    __device__ __forceinline__ static T w_bf(T q, T fac)
     {
-        const float t = fmaxf(fmaf(-0.5f, q, 1.0f), 0.0f);
-        const float t2 = t * t;
-        return fac * (t2 * t2 * fmaf(2.0f, q, 1.0f));
+        const T t = fmax(fma(T(-0.5), q, T(1)), T(0));
+        const T t2 = t * t;
+        return fac * (t2 * t2 * fma(T(2), q, T(1)));
     }
 
     // dW/dr / r = -5 q t^3 fac / (h r) = -5 t^3 fac / h^2
-    __device__ __forceinline__ static float gw_bf(float q, float, float ih, float fac_ih)
+    template <typename T>
+    __device__ __forceinline__ static T gw_bf(T q, T, T ih, T fac_ih)
     {
-        const float t = fmaxf(fmaf(-0.5f, q, 1.0f), 0.0f);
-        return fac_ih * ih * (-5.0f * (t * t * t));
-    }
-
-    template <int DIM>
-    __device__ __forceinline__ static double w_d(double rab, double h)
-    {
-        const double fac = norm<DIM>() * (1.0 / (h * h));
-        const double q = rab / h;
-        double val;
-        double tmp = __dsub_rn(1.0, __dmul_rn(0.5, q));
-        if (q > 2.0) {
-            val = 0.0;
-        } else {
-            tmp = __dmul_rn(tmp, __dmul_rn(__dmul_rn(tmp, tmp), tmp));
-            tmp = __dmul_rn(tmp, __dadd_rn(__dmul_rn(2.0, q), 1.0));
-            val = tmp;
-        }
-        return val * fac;
-    }
-
-    template <int DIM>
-    __device__ __forceinline__ static double gw_d(double rab, double h)
-    {
-        double fac = norm<DIM>() * (1.0 / (h * h));
-        const double q = rab / h;
-        double val;
-        double tmp = __dsub_rn(1.0, __dmul_rn(0.5, q));
-        if (rab < 1e-16) {
-            val = 0.0;
-        } else {
-            fac *= 1. / (h * rab);
-            if (q > 2.0) {
-                val = 0;
-            } else {
-                tmp = __dmul_rn(tmp, __dmul_rn(tmp, tmp));
-                val = __dmul_rn(__dmul_rn(tmp, -5.0), q);
-            }
-        }
-        return val * fac;
+        const T t = fmax(fma(T(-0.5), q, T(1)), T(0));
+        return fac_ih * ih * (T(-5) * (t * t * t));
     }
 };
 

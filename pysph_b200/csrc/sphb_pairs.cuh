@@ -230,6 +230,23 @@ __device__ __forceinline__ EntryF entry_unpack_f(uint32_t v)
     return r;
 }
 
+// The particle of a list entry of the FP64 passes, which take the absolute
+// positions and need no cell offset; false (j the dest itself, safe to load)
+// for a pad entry and, status flagged, for an index past the set.
+template <int DIM>
+__device__ __forceinline__ bool list_entry_d(const sphb_engine &e, uint32_t v, int k, int &j)
+{
+    constexpr int B = DIM == 2 ? SPHB_NBR_IDX_BITS_2D : SPHB_NBR_IDX_BITS_3D;
+    j = (int)(v & ((1u << B) - 1u));
+    bool ok = ((v >> B) & 7u) != 7u;
+    if (j >= e.cfg.num_particles) {
+        atomicOr(e.work.status, (unsigned)SPHB_ST_BAD_INDEX);
+        j = k;
+        ok = false;
+    }
+    return ok;
+}
+
 // Entries of dest k this lane owns (-1 when some lane's list overflowed),
 // or -1 when the lists are not to be used.
 template <int LANES>
@@ -253,8 +270,9 @@ __device__ __forceinline__ int list_count(const sphb_engine &e, bool use_list, i
 // next batch's list entries are fetched before this batch's records, so a
 // thread keeps U record gathers and U list loads in flight instead of one
 // dependent chain.  The last batch reads the list's pad entries (U divides
-// SPHB_LIST_PAD), which the neighbour test rejects.
-template <int DIM, int LANES, int U, typename Load, typename Use>
+// SPHB_LIST_PAD), which the FP32C neighbour test rejects and the FP64 load
+// knows by their offset field (list_entry_d).
+template <int LANES, int U, typename Load, typename Use>
 __device__ __forceinline__ void list_loop(const sphb_engine &e, int k, int lane, int cnt,
                                           Load &&load, Use &&use)
 {
@@ -273,9 +291,9 @@ __device__ __forceinline__ void list_loop(const sphb_engine &e, int k, int lane,
     for (int b = 0; b < nb; ++b) {
         uint32_t w[U];
         if (b + 1 < nb) fetch(b + 1, w);
-        decltype(load(EntryF{})) r[U];
+        decltype(load(0u)) r[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) r[u] = load(entry_unpack_f<DIM>(v[u]));
+        for (int u = 0; u < U; ++u) r[u] = load(v[u]);
 #pragma unroll
         for (int u = 0; u < U; ++u) use(r[u]);
 #pragma unroll

@@ -190,8 +190,15 @@ __device__ __forceinline__ void exchange_field(const sphb_engine &e, int cur, in
                               : field == 16 ? e.f.cs : field == 17 ? e.f.au
                               : field == 18 ? e.f.av : field == 19 ? e.f.aw
                               : e.f.dt_fac);
-        if (dir == 0) f[k] = user[ui];
-        else user[ui] = f[k];
+        if (dir == 0) {
+            f[k] = user[ui];
+            if (field <= 15 && e.f.thermo) {   // P / rho^2 follows rho and p
+                const double r = ((const double *)e.f.rho)[k];
+                ((double *)e.f.thermo)[k] = ((const double *)e.f.p)[k] * (1.0 / (r * r));
+            }
+        } else {
+            user[ui] = f[k];
+        }
     }
 }
 

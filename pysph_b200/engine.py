@@ -369,7 +369,8 @@ class Engine:
             for n in ("rho", "p", "cs", "au", "av", "dt_fac"):
                 f[n] = torch.zeros(N, **f64)
             f["aw"] = torch.zeros(N, **f64) if dim == 3 else None
-            f["geo"] = f["mass"] = f["vel"] = f["thermo"] = None
+            f["geo"] = f["mass"] = f["vel"] = None
+            f["thermo"] = torch.zeros(N, **f64)   # P / rho^2 for the force pass
             f["geo_next"] = f["vel_next"] = None
         f["cell"] = torch.zeros(N, **i32)
         # outputs of SPHDensityRate (_a_rho_1) and XSPHCorrection (velocity):
