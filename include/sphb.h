@@ -31,7 +31,7 @@ extern "C" {
 #endif
 
 #define SPHB_MAX_ARRAYS 4
-#define SPHB_ABI_VERSION 2
+#define SPHB_ABI_VERSION 3
 
 #if defined(__GNUC__)
 #define SPHB_API __attribute__((visibility("default")))
@@ -84,8 +84,8 @@ typedef struct {
     int32_t pair_block;     /* threads per block of the pair kernels, 32..256 */
     int32_t num_particles;  /* total over all segments */
     int32_t cell_capacity;  /* cell table capacity (all scenes, all arrays) */
-    int32_t list_batch;     /* list entries the FP32C force pass loads ahead
-                               per thread: 2 or 4 (0: 4) */
+    int32_t list_batch;     /* 0, 2 or 4; has no effect (the force pass loads
+                               two list entries ahead, the faster depth) */
     /* the scheme, per array index (identical for every scene):
      * SPHRho sources, MomentumEquation sources (bitmasks over arrays),
      * TaitEquation dests and integrated arrays (bitmasks) */
@@ -207,8 +207,8 @@ typedef struct {
     int32_t *cell;          /* local cell index of each particle */
     /* Neighbour lists of the last sphb_density pass (optional, may be
      * NULL): uint32 [list_cap][N] slot-major, entry = j | cell offsets
-     * (SPHB_NBR_* packing), and int32 [lanes][N] entries per lane (-1 when
-     * a lane overflowed its list_cap / lanes slots). */
+     * (SPHB_NBR_* packing), and int32 [N] entries of each list (-1 when it
+     * overflowed list_cap less a part of 4 x lanes slots). */
     uint32_t *nbr;
     int32_t *nbr_cnt;
     /* Optional (NULL: no list reuse across stages): FP32 position of every

@@ -98,7 +98,7 @@ BUFFER_FIELDS = ("x", "y", "z", "u", "v", "w", "x0", "y0", "z0", "u0", "v0",
                  "kx", "ky", "kz", "ku", "kv", "kw", "krho")
 
 
-ABI_VERSION = 2
+ABI_VERSION = 3
 
 
 class Buffers(ctypes.Structure):

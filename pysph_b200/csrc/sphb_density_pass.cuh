@@ -123,13 +123,10 @@ k_density(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask, in
     const int *__restrict__ start = e.work.start;
     unsigned int np = 0;   // pairs of this thread
     double rho = 0.0;
-    // neighbour list of this lane: slots lane, lane + LANES, ... of k,
-    // recorded (unless this pass reads them) with the skin when they are
-    // meant for reuse
+    // neighbour list of this dest, recorded (unless this pass reads them)
+    // with the skin when it is meant for reuse
     const int N = e.cfg.num_particles;
-    uint32_t *__restrict__ nbr = (e.f.list_cap > 0 && !from_list) ? e.f.nbr : nullptr;
-    // a lane's slots, whole pads of SPHB_LIST_PAD
-    const int cap_lane = (e.f.list_cap / LANES) & ~(SPHB_LIST_PAD - 1);
+    uint32_t *nbr = (e.f.list_cap > 0 && !from_list) ? e.f.nbr : nullptr;
     const double skin = (nbr && reuse) ? sc.skin_max : 0.0;
     if (nbr && blockIdx.x == 0 && threadIdx.x == 0) {
         // reusable only when recorded with the skin at the anchors (the
@@ -138,169 +135,193 @@ k_density(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask, in
         e.work.meta[4] = (reuse && e.work.meta[3] == 2) ? 1 : 0;
         if (!reuse) e.work.meta[2] = 0;
     }
-    int cnt = 0;
-    auto record = [&](int j, int o, int dy, int dz) {
-        if (nbr) {
-            if (cnt < cap_lane)
-                nbr[(size_t)(lane + LANES * cnt) * N + k] = nbr_pack<DIM>(j, o, dy, dz);
-            ++cnt;
-        }
-    };
+    int recorded = -1;   // entries of the list (-1: overflow, or none recorded)
 
+    extern __shared__ int2 s_rows[];   // record_list's row ranges
+    // FP32C in 2D with cells of the whole reach: summing while searching
+    // saves the second look at the lists (442 against 474 us, the recording
+    // pass of 256 drops); with cells of half the reach, in 3D, in FP64 and
+    // for the wide quintic the sum over the recorded list is shorter (3D
+    // cube of 64k 145 -> 93 us, FP64 dam break of 86k 38.6 -> 34.1 us,
+    // quintic drop of 50k 55.6 -> 50.0 us)
+    constexpr bool ONE_PHASE =
+        F32 && DIM == 2 && R == 1 && LANES == 1 && KT != SPHB_KERNEL_QUINTIC;
+    const int kq = active ? k : tl.begin;   // inactive threads read a valid particle
     if constexpr (F32) {
         Kahan acc;
+        const float4 *__restrict__ geo = (const float4 *)e.f.geo;
+        const float *__restrict__ mass = (const float *)e.f.mass;
+        const float4 gk = geo[kq];
+        const float csf = (float)sc.cell_size;
+        const float xk = gk.x, yk = gk.y, zk = DIM == 3 ? gk.z : 0.f;
+        const float hk = DIM == 3 ? gk.w : gk.z;
+        const float rad = hk * (float)sc.radius_scale;
+        const float rad2 = rad * rad;
+        // variable h: symmetric lists and, with hks, W averaged over h_a, h_b
+        const bool vh = sc.variable_h != 0, hks = sc.hks != 0;
+        const float rsf = (float)sc.radius_scale;
+        // a candidate of the list: within the support (the larger of the two
+        // with variable h) plus the skin
+        const float radl = (float)((hk * sc.radius_scale + skin) * (1.0 + 1e-5));
+        const float radl2 = radl * radl;
+        const float skinf = (float)skin;
+        auto listed = [&](float r2, float hj, bool sym) {
+            const float rl = (hj * rsf + skinf) * (1.0f + 1e-5f);
+            return r2 < (sym ? fmaxf(radl2, rl * rl) : radl2);
+        };
+        auto dist2_to = [&](const float4 &g, float o, float dy, float dz) {
+            const float dx = fmaf(-o, csf, xk - g.x);
+            const float ddy = fmaf(-dy, csf, yk - g.y);
+            float r2 = fmaf(ddy, ddy, mul_pair(dx, dx));
+            if (DIM == 3) {
+                const float ddz = fmaf(-dz, csf, zk - g.z);
+                r2 = fmaf(ddz, ddz, r2);
+            }
+            return r2;
+        };
+        if constexpr (LANES > 1) {
+            if (nbr) {
+                const int local = e.f.cell[kq];
+                int cx, cy, cz;
+                cell_coords(local, n, cx, cy, cz);
+                recorded = record_list<DIM, R, LANES>(
+                    e, nbr, s_rows, k, active, src, cell_base, ncells, n, local, cx, cy, cz,
+                    cell_trim_rel(e, xk, yk, zk, csf), [&](int j, int o, int dy, int dz) {
+                        const float4 g = __ldg(geo + j);
+                        return listed(dist2_to(g, (float)o, (float)dy, (float)dz),
+                                      DIM == 3 ? g.w : g.z, vh);
+                    });
+            }
+        }
         if (active) {
-            const float4 *__restrict__ geo = (const float4 *)e.f.geo;
-            const float *__restrict__ mass = (const float *)e.f.mass;
-            const float4 gk = geo[k];
-            const float csf = (float)sc.cell_size;
-            const float xk = gk.x, yk = gk.y, zk = DIM == 3 ? gk.z : 0.f;
-            const float hk = DIM == 3 ? gk.w : gk.z;
-            const float rad = hk * (float)sc.radius_scale;
-            const float rad2 = rad * rad;
-            const float radl = (float)((hk * sc.radius_scale + skin) * (1.0 + 1e-5));
-            const float radl2 = nbr ? radl * radl : rad2;
             const float kf = (float)Kern<KT>::template norm<DIM>();
-            const float ihk = __fdividef(1.0f, hk);
+            const float ihk = rcp_pair(hk);
             const float fack = DIM == 2 ? kf * ihk * ihk : kf * ihk * ihk * ihk;
-            // variable h: symmetric lists and, with hks, W averaged over h_a, h_b
-            const bool vh = sc.variable_h != 0, hks = sc.hks != 0;
-            const float rsf = (float)sc.radius_scale;
-            const float skinf = (float)skin;
             struct Rec {
                 float4 g;
-                float m, o, dy, dz;
+                float m;
                 bool ok;
             };
-            auto load = [&](const EntryF &en) {
+            // list entries index the set (pads the dest itself); the clamp
+            // only keeps a damaged list inside the arrays
+            auto load = [&](int j_) {
                 Rec r;
-                // list entries index the set (pads the dest itself); the
-                // clamp only keeps a damaged list inside the arrays
-                const int j = min(en.j, N - 1);
+                const int j = min(j_, N - 1);
                 r.ok = !filt || ((rsrc >> seg.array_of(j)) & 1u);
                 r.g = __ldg(geo + j);
                 r.m = DIM == 3 ? __ldg(mass + j) : r.g.w;
-                r.o = en.o;
-                r.dy = en.dy;
-                r.dz = en.dz;
                 return r;
-            };
-            auto dist2 = [&](const Rec &r) {
-                const float dx = (xk - r.g.x) - r.o * csf;
-                const float ddy = (yk - r.g.y) - r.dy * csf;
-                float r2 = dx * dx + ddy * ddy;
-                if (DIM == 3) {
-                    const float ddz = (zk - r.g.z) - r.dz * csf;
-                    r2 += ddz * ddz;
-                }
-                return r2;
             };
             // uniform h (every particle of the scene): h_ab = h_a, and the
             // kernel's 1/h and normalisation are the dest's
             auto pass = [&](auto uniform) {
                 constexpr bool UH = decltype(uniform)::value;
-                auto use = [&](const Rec &r, float r2) {
-                    if (lists_only || !r.ok) return;
+                // flat: the list loops' form, every entry evaluated and the
+                // ones outside the support adding 0 (list entries lie within
+                // the support plus the skin, so few do), which leaves no
+                // branch between the entries of a batch
+                auto use = [&](const Rec &r, float r2, auto flat) {
                     const float hj = DIM == 3 ? r.g.w : r.g.z;
-                    if (UH || !vh) {
-                        if (!(r2 < rad2)) return;
-                    } else {
+                    bool in = !lists_only && r.ok && r2 < rad2;
+                    if (!UH && vh) {
                         const float rj = hj * rsf;   // r < radius_scale max(h_a, h_b)
-                        if (!(r2 < rad2 || r2 < rj * rj)) return;
+                        in = !lists_only && r.ok && (r2 < rad2 || r2 < rj * rj);
                     }
+                    if (!decltype(flat)::value && !in) return;
                     const float ir = inv_dist(r2);   // q = 0 at r = 0
                     float w;
                     if (UH) {
-                        w = Kern<KT>::w_bf(r2 * ir * ihk, fack);
+                        w = Kern<KT>::template w_in<false>(mul_pair(r2 * ir, ihk), fack);
                     } else {
-                        // W(r, h_ab), or with hks (W(r, h_a) + W(r, h_b)) / 2; one
-                        // kernel evaluation in a loop keeps the register count
+                        // W(r, h_ab), or with hks (W(r, h_a) + W(r, h_b)) / 2
                         const float rr = r2 * ir;
-                        float hs = hks ? hk : 0.5f * (hk + hj);
-                        w = 0.f;
-#pragma unroll 1
-                        for (int t = 0;; ++t) {
-                            const float ih = __fdividef(1.0f, hs);
-                            const float fac = DIM == 2 ? kf * ih * ih : kf * ih * ih * ih;
-                            w += Kern<KT>::w_bf(rr * ih, fac);
-                            if (!hks || t == 1) break;
-                            hs = hj;
-                        }
-                        if (hks) w *= 0.5f;
+                        auto w_at = [&](float hs) {
+                            const float ih = rcp_pair(hs);
+                            return Kern<KT>::template w_in<true>(
+                                mul_pair(rr, ih), DIM == 2 ? kf * ih * ih : kf * ih * ih * ih);
+                        };
+                        w = hks ? 0.5f * (w_at(hk) + w_at(hj)) : w_at(0.5f * (hk + hj));
                     }
-                    acc.add(r.m * w);
-                    ++np;
+                    acc.add(in ? mul_pair(r.m, w) : 0.f);
+                    np += in;
                 };
                 // the common case (one h, every source summed, densities
                 // wanted) with the tests that cannot fail there out of the
                 // loops: the same arithmetic as load() and use()
                 const bool plain = UH && !filt && !lists_only;
-                auto load_all = [&](const EntryF &en) {
+                auto load_all = [&](int j_) {
                     Rec r;
-                    const int j = min(en.j, N - 1);
+                    const int j = min(j_, N - 1);
                     r.ok = true;
                     r.g = __ldg(geo + j);
                     r.m = DIM == 3 ? __ldg(mass + j) : r.g.w;
-                    r.o = en.o;
-                    r.dy = en.dy;
-                    r.dz = en.dz;
                     return r;
                 };
                 auto sum_plain = [&](const Rec &r, float r2) {
-                    if (r2 < rad2) {
-                        const float ir = inv_dist(r2);   // q = 0 at r = 0
-                        acc.add(r.m * Kern<KT>::w_bf(r2 * ir * ihk, fack));
-                        ++np;
-                    }
+                    const bool in = r2 < rad2;
+                    const float ir = inv_dist(r2);   // q = 0 at r = 0
+                    const float w = Kern<KT>::template w_in<false>(mul_pair(r2 * ir, ihk), fack);
+                    acc.add(in ? mul_pair(r.m, w) : 0.f);
+                    np += in;
                 };
-                const int lc = list_count<LANES>(e, from_list, k, lane);
-                if (lc >= 0) {
-                    if (plain) {
-                        list_loop<LANES, 4>(
-                            e, k, lane, lc,
-                            [&](uint32_t v) { return load_all(entry_unpack_f<DIM>(v)); },
-                            [&](const Rec &r) { sum_plain(r, dist2(r)); });
-                        return;
+                if constexpr (LANES == 1) {
+                    if (nbr) {
+                        // one thread a dest: record, then sum over the list
+                        // just written, whose entries are nearly all
+                        // neighbours (candidates are 15 to 50% of the time);
+                        // ONE_PHASE sums while it searches
+                        ListWriter<DIM, 1> list(nbr, k, e);
+                        int cx, cy, cz;
+                        cell_coords(e.f.cell[k], n, cx, cy, cz);
+                        for_each_candidate<DIM, R, 1>(
+                            start, A, src, cell_base, ncells, n, cx, cy, cz, lane, N,
+                            e.work.status, cell_trim_rel(e, xk, yk, zk, csf),
+                            [&](int j, int o, int dy, int dz) {
+                                const float4 g = __ldg(geo + j);
+                                const float r2 = dist2_to(g, (float)o, (float)dy, (float)dz);
+                                list.put(listed(r2, DIM == 3 ? g.w : g.z, !UH && vh), j, o, dy,
+                                         dz);
+                                if (ONE_PHASE) {
+                                    const Rec r{g, g.w, !filt || ((rsrc >> seg.array_of(j)) & 1u)};
+                                    use(r, r2, std::false_type{});
+                                }
+                            });
+                        recorded = list.finish(k);
+                        if (ONE_PHASE || lists_only) return;
                     }
-                    list_loop<LANES, 4>(
-                        e, k, lane, lc,
-                        [&](uint32_t v) { return load(entry_unpack_f<DIM>(v)); },
-                        [&](const Rec &r) { use(r, dist2(r)); });
+                }
+                if (lists_only) return;
+                // the list just recorded, or the kept one
+                const int cnt = nbr ? recorded : list_count(e, from_list, k);
+                if (cnt >= 0) {
+                    auto dist2 = [&](const Rec &r, uint32_t v) {
+                        const EntryF en = entry_unpack_f<DIM>(v);
+                        return dist2_to(r.g, en.o, en.dy, en.dz);
+                    };
+                    if (plain)
+                        list_loop<LANES, 4>(
+                            e, k, lane, cnt,
+                            [&](uint32_t v) { return load_all(entry_index<DIM>(v)); },
+                            [&](const Rec &r, uint32_t v) {
+                                sum_plain(r, dist2(r, v));
+                            });
+                    else
+                        list_loop<LANES, 4>(
+                            e, k, lane, cnt,
+                            [&](uint32_t v) { return load(entry_index<DIM>(v)); },
+                            [&](const Rec &r, uint32_t v) {
+                                use(r, dist2(r, v), std::true_type{});
+                            });
                     return;
                 }
                 int cx, cy, cz;
                 cell_coords(e.f.cell[k], n, cx, cy, cz);
-                if (plain && nbr) {
-                    // the recording pass of the common case
-                    for_each_candidate<DIM, R, LANES>(
-                        start, A, src, cell_base, ncells, n, cx, cy, cz, lane, N, e.work.status,
-                        cell_trim_rel(e, xk, yk, zk, csf), [&](int j, int o, int dy, int dz) {
-                            const Rec r = load_all(EntryF{j, (float)o, (float)dy, (float)dz});
-                            const float r2 = dist2(r);
-                            if (r2 < radl2) {
-                                if (cnt < cap_lane)
-                                    nbr[(size_t)(lane + LANES * cnt) * N + k] =
-                                        nbr_pack<DIM>(j, o, dy, dz);
-                                ++cnt;
-                            }
-                            sum_plain(r, r2);
-                        });
-                    return;
-                }
                 for_each_candidate<DIM, R, LANES>(
                     start, A, src, cell_base, ncells, n, cx, cy, cz, lane, N, e.work.status,
                     cell_trim_rel(e, xk, yk, zk, csf), [&](int j, int o, int dy, int dz) {
-                        const Rec r = load(EntryF{j, (float)o, (float)dy, (float)dz});
-                        const float r2 = dist2(r);
-                        bool rec = r2 < radl2;
-                        if (!UH && vh && nbr && !rec) {
-                            // the larger of the two supports, with the skin
-                            const float hj = DIM == 3 ? r.g.w : r.g.z;
-                            const float rl = (hj * rsf + skinf) * (1.0f + 1e-5f);
-                            rec = hj > hk && r2 < rl * rl;
-                        }
-                        if (rec) record(j, o, dy, dz);
-                        use(r, r2);
+                        const Rec r = load(j);
+                        use(r, dist2_to(r.g, (float)o, (float)dy, (float)dz),
+                            std::false_type{});
                     });
             };
             if (sc.uniform_h) pass(std::true_type{});
@@ -315,20 +336,50 @@ k_density(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask, in
         rho = acc.value();
     } else {
         double sum = 0.0;
-        if (active) {
-            const sphb_buffers &B = e.buf[cur];
-            const double xk = B.x[k], yk = B.y[k], zk = DIM == 3 ? B.z[k] : 0.0;
-            const double hk = B.h[k];
-            const double rad = hk * sc.radius_scale;
-            const double rad2 = __dmul_rn(rad, rad);
-            const double radl = (rad + skin) * (1.0 + 1e-5);
-            const double radl2 = nbr ? radl * radl : rad2;
+        const sphb_buffers &B = e.buf[cur];
+        const double xk = B.x[kq], yk = B.y[kq], zk = DIM == 3 ? B.z[kq] : 0.0;
+        const double hk = B.h[kq];
+        const double rad = hk * sc.radius_scale;
+        const double rad2 = __dmul_rn(rad, rad);
+        // with one h in the scene the symmetric set and the averaged kernel
+        // are the plain ones
+        const bool vh = sc.variable_h != 0, hks = sc.hks != 0;
+        const double radl = (rad + skin) * (1.0 + 1e-5);
+        const double radl2 = radl * radl;
+        auto accept = [&](int j, auto sym) {
+            const double d2 = dist2_ref<DIM>(xk - __ldg(B.x + j), yk - __ldg(B.y + j),
+                                             DIM == 3 ? zk - __ldg(B.z + j) : 0.0);
+            if (!decltype(sym)::value) return d2 < radl2;
+            const double rl = (__ldg(B.h + j) * sc.radius_scale + skin) * (1.0 + 1e-5);
+            return d2 < fmax(radl2, rl * rl);
+        };
+        auto record = [&](auto sym) {
+            const int local = e.f.cell[kq];
+            int cx, cy, cz;
+            cell_coords(local, n, cx, cy, cz);
+            const CellTrim trim = cell_trim_abs<DIM>(e, st, sc.cell_size, xk, yk, zk, cx, cy, cz);
+            if constexpr (LANES > 1) {
+                recorded = record_list<DIM, R, LANES>(
+                    e, nbr, s_rows, k, active, src, cell_base, ncells, n, local, cx, cy, cz, trim,
+                    [&](int j, int, int, int) { return accept(j, sym); });
+            } else if (active) {
+                ListWriter<DIM, 1> list(nbr, k, e);
+                for_each_candidate<DIM, R, 1>(
+                    start, A, src, cell_base, ncells, n, cx, cy, cz, lane, N, e.work.status, trim,
+                    [&](int j, int o, int oy, int oz) {
+                        list.put(accept(j, sym), j, o, oy, oz);
+                    });
+                recorded = list.finish(k);
+            }
+        };
+        if (nbr) {   // block-uniform, as is what the scene says of h
+            if (vh && !sc.uniform_h) record(std::true_type{});
+            else record(std::false_type{});
+        }
+        if (active && !(lists_only && nbr)) {
             const double kf = Kern<KT>::template norm<DIM>();
             const double ihk = 1.0 / hk;
             const double fack = DIM == 2 ? kf * ihk * ihk : kf * ihk * ihk * ihk;
-            // with one h in the scene the symmetric set and the averaged
-            // kernel are the plain ones
-            const bool vh = sc.variable_h != 0, hks = sc.hks != 0;
             struct Rec {
                 double x, y, z, m, h;
                 bool ok;
@@ -348,46 +399,42 @@ k_density(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask, in
                 auto dist2 = [&](const Rec &r) {
                     return dist2_ref<DIM>(xk - r.x, yk - r.y, DIM == 3 ? zk - r.z : 0.0);
                 };
-                auto use = [&](const Rec &r, double d2) {
+                auto use = [&](const Rec &r, double d2, auto flat) {
                     // symmetric: r^2 < (radius_scale h_a)^2 or (radius_scale h_b)^2
                     double radj2 = rad2;
                     if (!UH && vh) {
                         const double rj = r.h * sc.radius_scale;
                         radj2 = fmax(rad2, __dmul_rn(rj, rj));
                     }
-                    if (!r.ok || !(d2 < radj2)) return;
+                    const bool in = r.ok && d2 < radj2;
+                    if (!decltype(flat)::value && !in) return;
                     const double ir = inv_dist(d2);
                     double w;
                     if (UH) {
-                        w = Kern<KT>::w_bf(d2 * ir * ihk, fack);
+                        w = Kern<KT>::template w_in<false>(mul_pair(d2 * ir, ihk), fack);
                     } else {
                         // W(r, h_ab), or with hks (W(r, h_a) + W(r, h_b)) / 2
                         const double rr = d2 * ir;
-                        double hs = hks ? hk : 0.5 * (hk + r.h);
-                        w = 0.0;
-#pragma unroll 1
-                        for (int t = 0;; ++t) {
-                            const double ih = 1.0 / hs;
-                            w += Kern<KT>::w_bf(rr * ih,
-                                                DIM == 2 ? kf * ih * ih : kf * ih * ih * ih);
-                            if (!hks || t == 1) break;
-                            hs = r.h;
-                        }
-                        if (hks) w *= 0.5;
+                        auto w_at = [&](double hs) {
+                            const double ih = rcp_pair(hs);
+                            return Kern<KT>::template w_in<true>(
+                                mul_pair(rr, ih), DIM == 2 ? kf * ih * ih : kf * ih * ih * ih);
+                        };
+                        w = hks ? 0.5 * (w_at(hk) + w_at(r.h)) : w_at(0.5 * (hk + r.h));
                     }
-                    sum += r.m * w;
-                    ++np;
+                    sum += in ? r.m * w : 0.0;
+                    np += in;
                 };
-                const int lc = list_count<LANES>(e, from_list, k, lane);
-                if (lc >= 0) {
+                const int cnt = nbr ? recorded : list_count(e, from_list, k);
+                if (cnt >= 0) {
                     list_loop<LANES, 4>(
-                        e, k, lane, lc,
+                        e, k, lane, cnt,
                         [&](uint32_t v) {
                             int j;
                             const bool ok = list_entry_d<DIM>(e, v, k, j);
                             return load(j, ok);
                         },
-                        [&](const Rec &r) { use(r, dist2(r)); });
+                        [&](const Rec &r, uint32_t) { use(r, dist2(r), std::true_type{}); });
                     return;
                 }
                 int cx, cy, cz;
@@ -395,16 +442,9 @@ k_density(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask, in
                 for_each_candidate<DIM, R, LANES>(
                     start, A, src, cell_base, ncells, n, cx, cy, cz, lane, N, e.work.status,
                     cell_trim_abs<DIM>(e, st, sc.cell_size, xk, yk, zk, cx, cy, cz),
-                    [&](int j, int o, int oy, int oz) {
-                        const Rec r = load(j, !lists_only);
-                        const double d2 = dist2(r);
-                        bool rec = d2 < radl2;
-                        if (!UH && vh && nbr && !rec) {
-                            const double rl = (r.h * sc.radius_scale + skin) * (1.0 + 1e-5);
-                            rec = r.h > hk && d2 < rl * rl;
-                        }
-                        if (rec) record(j, o, oy, oz);
-                        use(r, d2);
+                    [&](int j, int, int, int) {
+                        const Rec r = load(j, true);
+                        use(r, dist2(r), std::false_type{});
                     });
             };
             if (sc.uniform_h) pass(std::true_type{});
@@ -415,15 +455,7 @@ k_density(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask, in
         rho = sum;
     }
 
-    if (active && nbr) {
-        const int c_ok = cnt <= cap_lane ? cnt : -1;
-        if (c_ok >= 0) {
-            const int c_end = (c_ok + SPHB_LIST_PAD - 1) & ~(SPHB_LIST_PAD - 1);
-            for (int c = c_ok; c < c_end; ++c)
-                nbr[(size_t)(lane + LANES * c) * N + k] = nbr_pad<DIM>(k);
-        }
-        e.f.nbr_cnt[(size_t)lane * N + k] = c_ok;
-    }
+    if (active && nbr && lane == 0) e.f.nbr_cnt[k] = recorded;
     density_finish<F32>(e, cur, k, s, a, active && !lists_only, lane, rho, with_eos, np);
 }
 
@@ -432,7 +464,10 @@ static void launch_density_p(const sphb_engine &e, int cur, uint32_t dm, int eos
                              cudaStream_t st)
 {
     const dim3 g(e.num_pair_tiles), b(e.cfg.pair_block);
-#define SPHB_L(LV, RV) launch_pdl(k_density<KT, DIM, F32, LV, RV>, g, b, st, e, cur, dm, eos)
+#define SPHB_L(LV, RV)                                                                   \
+    launch_pdl(k_density<KT, DIM, F32, LV, RV>, g, b,                                    \
+               e.f.list_cap > 0 ? record_smem<DIM, RV, LV>(e.cfg.pair_block) : 0, st, e, \
+               cur, dm, eos)
     switch (e.cfg.lanes * 10 + e.cfg.stencil) {
     case 11: SPHB_L(1, 1); break;
     case 12: SPHB_L(1, 2); break;

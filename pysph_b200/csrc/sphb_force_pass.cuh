@@ -131,29 +131,31 @@ __device__ __forceinline__ void force_finish(const sphb_engine &e, int cur, int 
     block_add_u64(&e.work.pairs[1], np);
 }
 
-// List entries the FP64 force pass loads ahead.  The FP64 pair was bound by
-// its own latency: one neighbour at a time, four dependent rounds of loads
-// (position; h, rho, p, m; velocity; cs) and eight divisions and a square
-// root in branches.  With every field of a batch loaded up front, P / rho^2
-// kept per particle, one reciprocal square root and the dest's 1 / h instead
-// of the kernel's divisions, the pass with the density pass it overlaps goes
-// 134 -> 63 us on an 86k-particle 2D dam break and 95 -> 40 us on a 5k drop
-// (one lane per particle); batches of 4 do not fit 128 registers.
-constexpr int FP64_BATCH = 2;
-
 // CONT: the continuity scheme's pair terms too -- SPHDensityRate
 // (density_funcs.pyx:119-156) and XSPHCorrection (xsph_funcs.pyx:40-86),
 // each over its own sources, in the same traversal as the momentum.
-// The 2D FP32C momentum-only variants are held to 80 registers (three
-// 256-thread blocks per SM) with list batches of 4, and to 64 (four blocks)
-// with batches of 2, which then need no spills: on the dam break the
-// latter's pass is 3% shorter (51.6 against 53.4 us), while batches of 4
-// at 64 registers spill 256 B and take 67.5 us.  Left alone, the fused
-// stage in the epilogue would take them to 96 (two blocks).  Every other
-// variant is held to 128 (two blocks): the FP64 continuity pass would
-// otherwise take 132 and fit one block per SM.
-template <int KT, int DIM, bool F32, int LANES, int R, int U, bool CONT>
-__global__ void __launch_bounds__(256, (F32 && !CONT && DIM == 2) ? (U == 2 ? 4 : 3) : 2)
+// Register bounds, the list loops two entries ahead (four, or the records
+// a batch ahead, lost at every bound; times of the pass with the density
+// pass it overlaps): FP32C in 2D 72 (seven 128-thread blocks per SM; 332k
+// dam break 3,778 us per 20 steps, 80 registers 3,966, 64 3,982; 256 drops
+// 377 us a pass, 80 registers 418, 64 366), in 3D 80 (128^3 lattice's pressure
+// gradient 597 us, 96 registers 671, 128 758), with the continuity terms 96
+// (1,109 us per 10 steps of 146k particles, 80 registers 1,122, 128 1,163).
+// FP64 in 2D 96: 16% of its 128-register time on an 86k-particle dam break
+// was a second wave of blocks (1,304 -> 1,248 us per 10 steps).
+// The FP64 pair was bound by its own latency: one neighbour at a time, four
+// dependent rounds of loads, eight divisions and a square root in branches.
+// With a batch's fields loaded together, P / rho^2 kept per particle, and no
+// division or branch in a pair, the pass goes 134 -> 42 us on that dam break.
+template <int DIM, bool F32, bool CONT>
+constexpr int force_regs()
+{
+    return F32 ? (CONT ? (DIM == 3 ? 128 : 96) : (DIM == 2 ? 72 : 80))
+               : (DIM == 2 && !CONT ? 96 : 128);
+}
+
+template <int KT, int DIM, bool F32, int LANES, int R, bool CONT>
+__global__ void __maxnreg__((force_regs<DIM, F32, CONT>()))
 k_force(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask,
         int with_gravity, int mode)
 {
@@ -197,7 +199,7 @@ k_force(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask,
     if constexpr (F32) {
         Kahan ax, ay, az;
         Kahan kr, kxx, kxy, kxz;   // density rate, XSPH velocity (CONT)
-        float dtmax = 0.f;
+        float dtmax = 0.f, dt_h = 1.0f;   // dt_fac = dtmax dt_h
         if (active) {
             const int N = e.cfg.num_particles;
             const float4 *__restrict__ geo = (const float4 *)e.f.geo;
@@ -224,26 +226,25 @@ k_force(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask,
             const float alpha = (float)sc.alpha, beta = (float)sc.beta;
             const float eta2 = (float)(sc.eta * sc.eta);
             const float kf = (float)Kern<KT>::template norm<DIM>();
-            const float ihk = __fdividef(1.0f, hk);
+            const float ihk = rcp_pair(hk);
             // fac / h of the dest: 2D kf/h^3, 3D kf/h^4
             const float fihk = DIM == 2 ? kf * ihk * ihk * ihk : kf * ihk * ihk * ihk * ihk;
-            const float eh2k = eta2 * hk * hk;
+            const float eh2k = mul_pair(eta2 * hk, hk);
+            const float alp_k = alpha * hk, bet2_k = 2.0f * beta * hk * hk;
             // variable h: symmetric lists and, with hks, W and grad W
             // averaged over h_a and h_b (the AV and the CFL keep h_ab)
             const bool vh = sc.variable_h != 0, hks = sc.hks != 0;
             const float rsf = (float)sc.radius_scale;
             struct Rec {
                 float4 g, t;
-                float vx, vy, vz, m, o, dy, dz;
+                float vx, vy, vz, m;
                 uint32_t bit;   // the source's array as a mask bit (CONT)
-                bool ok;
             };
-            auto load = [&](const EntryF &en) {
+            auto load = [&](int j_) {
                 Rec r;
                 // list entries index the set (pads the dest itself); the
                 // clamp only keeps a damaged list inside the arrays
-                const int j = min(en.j, N - 1);
-                r.ok = true;
+                const int j = min(j_, N - 1);
                 r.bit = filt ? 1u << seg.array_of(j) : ~0u;
                 r.g = __ldg(geo + j);
                 r.t = __ldg(th + j);
@@ -263,52 +264,53 @@ k_force(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask,
                 } else {
                     r.vx = r.vy = r.vz = 0.f;
                 }
-                r.o = en.o;
-                r.dy = en.dy;
-                r.dz = en.dz;
                 return r;
             };
             auto pass = [&](auto uniform) {
                 constexpr bool UH = decltype(uniform)::value;
+                if (UH) dt_h = hk;
                 // the pair body; with the force mode known at compile time
                 // (KM = 0 MomentumEquation, 1 SPHPressureGradient, 2 the
                 // split viscosity; -1 read at run time) the list loop
                 // carries no test of it
+                // The list loops (KM >= 0) evaluate every entry and have the
+                // ones outside the support add 0 (list entries lie within the
+                // support plus the skin, so few do): no branch separates the
+                // entries of a batch.  The cell search branches.
                 auto make_use = [&](auto known) {
                     constexpr int KM = decltype(known)::value;
                     const bool visc_k = KM < 0 ? visc : KM == 0;
                     const bool avisc_k = KM < 0 ? avisc : KM == 2;
-                    return [&, visc_k, avisc_k](const Rec &r) {
-                        const float rx = (xk - r.g.x) - r.o * csf;
-                        const float ry = (yk - r.g.y) - r.dy * csf;
+                    return [&, visc_k, avisc_k](const Rec &r, float o, float dy, float dz) {
+                        const float rx = fmaf(-o, csf, xk - r.g.x);
+                        const float ry = fmaf(-dy, csf, yk - r.g.y);
                         float rz = 0.f;
-                        float r2 = rx * rx + ry * ry;
+                        float r2 = fmaf(ry, ry, mul_pair(rx, rx));
                         if (DIM == 3) {
-                            rz = (zk - r.g.z) - r.dz * csf;
-                            r2 += rz * rz;
+                            rz = fmaf(-dz, csf, zk - r.g.z);
+                            r2 = fmaf(rz, rz, r2);
                         }
-                        if (!r.ok) return;
                         const float hj = DIM == 3 ? r.g.w : r.g.z;
-                        if (UH || !vh) {
-                            if (!(r2 < rad2)) return;
-                        } else {
+                        bool in = r2 < rad2;
+                        if (!UH && vh) {
                             const float rj = hj * rsf;   // r < radius_scale max(h_a, h_b)
-                            if (!(r2 < rad2 || r2 < rj * rj)) return;
+                            in = r2 < rad2 || r2 < rj * rj;
                         }
-                        ++np;
-                        const bool mom_on = !CONT || (mm & r.bit);
-                        const bool rate_on = CONT && (rm & r.bit);
-                        const bool xs_on = CONT && (xm & r.bit);
+                        if (KM < 0 && !in) return;
+                        np += in;
+                        const bool mom_on = in && (!CONT || (mm & r.bit));
+                        const bool rate_on = in && CONT && (rm & r.bit);
+                        const bool xs_on = in && CONT && (xm & r.bit);
                         float hab = hk, eh2 = eh2k;
                         if (!UH) {
                             hab = 0.5f * (hk + hj);
-                            eh2 = eta2 * hab * hab;
+                            eh2 = mul_pair(eta2 * hab, hab);
                         }
                         // P_a/rho_a^2 + P_b/rho_b^2 (none in the split viscosity)
                         float tmp = avisc_k ? 0.f : tk.w + r.t.w;
                         const float vx = uk - r.vx, vy = vk - r.vy, vz = wk - r.vz;
-                        float dot = vx * rx + vy * ry;
-                        if (DIM == 3) dot += vz * rz;
+                        float dot = fmaf(vy, ry, mul_pair(vx, rx));
+                        if (DIM == 3) dot = fmaf(vz, rz, dot);
                         // r = 0 (self) gives q = 0 and a finite gradient times r_ab = 0
                         const float ir = inv_dist(r2);
                         // grad W / r (and W for XSPH) at h_ab, or with hks the means
@@ -316,76 +318,77 @@ k_force(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask,
                         // keeps the register count of the uniform-h path
                         float gw, w = 0.f;
                         if (UH) {
-                            const float q = r2 * ir * ihk;
-                            gw = Kern<KT>::gw_bf(q, ir, ihk, fihk);
-                            if (CONT && xs_on) w = Kern<KT>::w_bf(q, fihk * hk);
+                            const float q = mul_pair(r2 * ir, ihk);
+                            gw = Kern<KT>::template gw_in<false>(q, ir, ihk, fihk);
+                            if (CONT) w = Kern<KT>::template w_in<false>(q, fihk * hk);
                         } else {
                             const float rr = r2 * ir;
-                            float hs = hks ? hk : hab;
-                            gw = 0.f;
-    #pragma unroll 1
-                            for (int t = 0;; ++t) {
-                                const float ih = __fdividef(1.0f, hs);
+                            auto at = [&](float hs, float &wh) {
+                                const float ih = rcp_pair(hs);
                                 const float fih = DIM == 2 ? kf * ih * ih * ih : kf * ih * ih * ih * ih;
-                                const float q = rr * ih;
-                                gw += Kern<KT>::gw_bf(q, ir, ih, fih);
-                                if (CONT && xs_on) w += Kern<KT>::w_bf(q, fih * hs);
-                                if (!hks || t == 1) break;
-                                hs = hj;
-                            }
+                                const auto q = mul_pair(rr, ih);
+                                if (CONT) wh = Kern<KT>::template w_in<true>(q, fih * hs);
+                                return Kern<KT>::template gw_in<true>(q, ir, ih, fih);
+                            };
+                            float wa = 0.f, wb = 0.f;
                             if (hks) {
-                                gw *= 0.5f;
-                                w *= 0.5f;
+                                gw = 0.5f * (at(hk, wa) + at(hj, wb));
+                                w = 0.5f * (wa + wb);
+                            } else {
+                                gw = at(hab, w);
                             }
                         }
                         if (CONT) {
                             // drho_a += m_b (v_a - v_b) . grad_a W
-                            if (rate_on) kr.add(r.m * (dot * gw));
+                            kr.add(rate_on ? mul_pair(r.m, dot * gw) : 0.f);
                             // XSPH: eps m_b W_ab (v_b - v_a) / rho_ab (eps at the end)
-                            if (xs_on) {
-                                const float temp = __fdividef(r.m * w, 0.5f * (tk.x + r.t.x));
-                                kxx.add(-temp * vx);
-                                kxy.add(-temp * vy);
-                                if (DIM == 3) kxz.add(-temp * vz);
-                            }
-                            if (!mom_on) return;
+                            const float temp = r.m * w * rcp_pair(0.5f * (tk.x + r.t.x));
+                            kxx.add(xs_on ? mul_pair(-temp, vx) : 0.f);
+                            kxy.add(xs_on ? mul_pair(-temp, vy) : 0.f);
+                            if (DIM == 3) kxz.add(xs_on ? mul_pair(-temp, vz) : 0.f);
                         }
                         if (visc_k || avisc_k) {
-                            const float mu = __fdividef(hab * dot, r2 + eh2);
+                            // mu / h_ab = dot / (r^2 + eta^2 h_ab^2); the factors
+                            // h_ab go into alpha and beta
+                            const float mu = dot * rcp_pair(r2 + eh2);
+                            const float alp = UH ? alp_k : alpha * hab;
+                            const float bet2 = UH ? bet2_k : 2.0f * beta * hab * hab;
                             // the split viscosity's dt_fac has 0.01 h_ab^2 written in
                             // (viscosity_funcs.pyx:103) whatever its eta
-                            dtmax = fmaxf(dtmax, fabsf(avisc_k ? __fdividef(hab * dot,
-                                                                           r2 + 0.01f * hab * hab)
-                                                             : mu));
+                            const float md =
+                                avisc_k ? dot * rcp_pair(r2 + 0.01f * hab * hab) : mu;
+                            dtmax = fmaxf(dtmax, mom_on ? fabsf(UH ? md : md * hab) : 0.f);
                             // Monaghan Pi_ab = (-alpha c_ab mu + beta mu^2) / rho_ab
                             // when v_ab . r_ab < 0, i.e. mu < 0; else 0: min(mu, 0)
+                            // (the halves of c_ab and rho_ab cancel)
                             const float mn = fminf(mu, 0.f);
-                            const float cab = 0.5f * (tk.z + r.t.z);
-                            const float rhoab = 0.5f * (tk.x + r.t.x);
-                            tmp += __fdividef(-alpha * cab * mn + beta * mn * mn, rhoab);
+                            const float c2 = tk.z + r.t.z, rho2 = tk.x + r.t.x;
+                            tmp = fmaf(mn * fmaf(bet2, mn, mul_pair(-alp, c2)), rcp_pair(rho2),
+                                       tmp);
                         }
+                        // (the products are selected, so a NaN outside the
+                        // support stays there)
                         const float f = -r.m * tmp * gw;
-                        ax.add(f * rx);
-                        ay.add(f * ry);
-                        if (DIM == 3) az.add(f * rz);
+                        ax.add(mom_on ? mul_pair(f, rx) : 0.f);
+                        ay.add(mom_on ? mul_pair(f, ry) : 0.f);
+                        if (DIM == 3) az.add(mom_on ? mul_pair(f, rz) : 0.f);
                     };
                 };
-                auto load_entry = [&](uint32_t v) { return load(entry_unpack_f<DIM>(v)); };
-                const int lc = list_count<LANES>(e, use_list, k, lane);
+                const int lc = list_count(e, use_list, k);
                 if (lc >= 0) {
+                    auto from_list = [&](auto known) {
+                        auto use = make_use(known);
+                        list_loop<LANES, 2>(
+                            e, k, lane, lc, [&](uint32_t v) { return load(entry_index<DIM>(v)); },
+                            [&](const Rec &r, uint32_t v) {
+                                const EntryF en = entry_unpack_f<DIM>(v);
+                                use(r, en.o, en.dy, en.dz);
+                            });
+                    };
                     switch (mode & 15) {   // block-uniform
-                    case 0:
-                        list_loop<LANES, U>(e, k, lane, lc, load_entry,
-                                            make_use(std::integral_constant<int, 0>{}));
-                        break;
-                    case 1:
-                        list_loop<LANES, U>(e, k, lane, lc, load_entry,
-                                            make_use(std::integral_constant<int, 1>{}));
-                        break;
-                    default:
-                        list_loop<LANES, U>(e, k, lane, lc, load_entry,
-                                            make_use(std::integral_constant<int, 2>{}));
-                        break;
+                    case 0: from_list(std::integral_constant<int, 0>{}); break;
+                    case 1: from_list(std::integral_constant<int, 1>{}); break;
+                    default: from_list(std::integral_constant<int, 2>{}); break;
                     }
                     return;
                 }
@@ -394,8 +397,9 @@ k_force(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask,
                 cell_coords(e.f.cell[k], n, cx, cy, cz);
                 for_each_candidate<DIM, R, LANES>(
                     start, A, src, cell_base, ncells, n, cx, cy, cz, lane, N, e.work.status,
-                    cell_trim_rel(e, xk, yk, zk, csf), [&](int j, int o, int dy, int dz) {
-                        use(load(EntryF{j, (float)o, (float)dy, (float)dz}));
+                    cell_trim_rel(e, xk, yk, zk, csf),
+                    [&](int j, int o, int dy, int dz) {
+                        use(load(j), (float)o, (float)dy, (float)dz);
                     });
             };
             if (sc.uniform_h) pass(std::true_type{});
@@ -412,7 +416,7 @@ k_force(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask,
         acc[0] = ax.value();
         acc[1] = ay.value();
         acc[2] = az.value();
-        dtf = dtmax;
+        dtf = dtmax * dt_h;
         if (CONT) {
 #pragma unroll
             for (int o = LANES / 2; o > 0; o >>= 1) {
@@ -429,6 +433,7 @@ k_force(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask,
             xs[2] = kxz.value() * sc.xsph_eps;
         }
     } else {
+        double dt_h = 1.0;
         if (active) {
             const int N = e.cfg.num_particles;
             const sphb_buffers &B = e.buf[cur];
@@ -452,6 +457,7 @@ k_force(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask,
             const double rad2 = __dmul_rn(rad, rad);
             const double alpha = sc.alpha, beta = sc.beta, eta2 = sc.eta * sc.eta;
             const double kf = Kern<KT>::template norm<DIM>();
+            const double alp_k = alpha * hk, bet2_k = 2.0 * beta * hk * hk;
             const double ihk = 1.0 / hk;
             const double fihk = DIM == 2 ? kf * ihk * ihk * ihk : kf * ihk * ihk * ihk * ihk;
             // with one h in the scene the symmetric set and the averaged
@@ -464,6 +470,7 @@ k_force(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask,
             };
             auto pass = [&](auto uniform) {
                 constexpr bool UH = decltype(uniform)::value;
+                if (UH) dt_h = hk;
                 // KM as in the FP32C body: the mode known at compile time in
                 // the list loops, -1 in the cell search
                 auto make_load = [&](auto known) {
@@ -503,11 +510,12 @@ k_force(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask,
                             const double rj = r.h * sc.radius_scale;
                             radj2 = fmax(rad2, __dmul_rn(rj, rj));
                         }
-                        if (!r.ok || !(r2 < radj2)) return;
-                        ++np;
-                        const bool mom_on = !CONT || (mm & r.bit);
-                        const bool rate_on = CONT && (rm & r.bit);
-                        const bool xs_on = CONT && (xm & r.bit);
+                        const bool in = r.ok && r2 < radj2;
+                        if (KM < 0 && !in) return;
+                        np += in;
+                        const bool mom_on = in && (!CONT || (mm & r.bit));
+                        const bool rate_on = in && CONT && (rm & r.bit);
+                        const bool xs_on = in && CONT && (xm & r.bit);
                         const double hab = UH ? hk : 0.5 * (hk + r.h);
                         const double ir = inv_dist(r2);
                         // grad W / r (and W for XSPH) at h_ab, or with hks the
@@ -515,47 +523,40 @@ k_force(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask,
                         // 371-381)
                         double gw, w = 0.0;
                         if (UH) {
-                            const double q = r2 * ir * ihk;
-                            gw = Kern<KT>::gw_bf(q, ir, ihk, fihk);
-                            if (CONT && xs_on) w = Kern<KT>::w_bf(q, fihk * hk);
+                            const double q = mul_pair(r2 * ir, ihk);
+                            gw = Kern<KT>::template gw_in<false>(q, ir, ihk, fihk);
+                            if (CONT) w = Kern<KT>::template w_in<false>(q, fihk * hk);
                         } else {
                             const double rr = r2 * ir;
-                            double hs = hks ? hk : hab;
-                            gw = 0.0;
-#pragma unroll 1
-                            for (int t = 0;; ++t) {
-                                const double ih = 1.0 / hs;
+                            auto at = [&](double hs, double &wh) {
+                                const double ih = rcp_pair(hs);
                                 const double fih = DIM == 2 ? kf * ih * ih * ih
                                                             : kf * ih * ih * ih * ih;
-                                const double q = rr * ih;
-                                gw += Kern<KT>::gw_bf(q, ir, ih, fih);
-                                if (CONT && xs_on) w += Kern<KT>::w_bf(q, fih * hs);
-                                if (!hks || t == 1) break;
-                                hs = r.h;
-                            }
+                                const auto q = mul_pair(rr, ih);
+                                if (CONT) wh = Kern<KT>::template w_in<true>(q, fih * hs);
+                                return Kern<KT>::template gw_in<true>(q, ir, ih, fih);
+                            };
+                            double wa = 0.0, wb = 0.0;
                             if (hks) {
-                                gw *= 0.5;
-                                w *= 0.5;
+                                gw = 0.5 * (at(hk, wa) + at(r.h, wb));
+                                w = 0.5 * (wa + wb);
+                            } else {
+                                gw = at(hab, w);
                             }
                         }
                         const double gx = rx * gw, gy = ry * gw, gz = rz * gw;
                         const double vx = uk - r.u, vy = vk - r.v, vz = wk - r.w;
                         if (CONT) {
-                            if (rate_on) {
-                                // SPHDensityRate: ((v_a - v_b) . grad_a W) m_b
-                                double d = vx * gx + vy * gy;
-                                if (DIM == 3) d += vz * gz;
-                                drho += d * r.m;
-                            }
-                            if (xs_on) {
-                                // XSPHCorrection: m_b W_ab / rho_ab (v_b - v_a) eps
-                                const double temp =
-                                    r.m * w / (0.5 * (r.rho + rhoa)) * sc.xsph_eps;
-                                xs[0] -= temp * vx;
-                                xs[1] -= temp * vy;
-                                if (DIM == 3) xs[2] -= temp * vz;
-                            }
-                            if (!mom_on) return;
+                            // SPHDensityRate: ((v_a - v_b) . grad_a W) m_b
+                            double d = vx * gx + vy * gy;
+                            if (DIM == 3) d += vz * gz;
+                            drho += rate_on ? d * r.m : 0.0;
+                            // XSPHCorrection: m_b W_ab / rho_ab (v_b - v_a) eps
+                            const double temp =
+                                r.m * w * rcp_pair(0.5 * (r.rho + rhoa)) * sc.xsph_eps;
+                            xs[0] -= xs_on ? temp * vx : 0.0;
+                            xs[1] -= xs_on ? temp * vy : 0.0;
+                            if (DIM == 3) xs[2] -= xs_on ? temp * vz : 0.0;
                         }
                         // P_a/rho_a^2 + P_b/rho_b^2; the split viscosity has none
                         // (tmp = piab; tmp *= -mb, viscosity_funcs.pyx:125-126)
@@ -563,33 +564,36 @@ k_force(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask,
                         if (visc_k || avisc_k) {
                             double dot = vx * rx + vy * ry;
                             if (DIM == 3) dot += vz * rz;
-                            const double hd = hab * dot;
-                            const double mu = hd / (r2 + eta2 * hab * hab);
-                            dtf = fmax(dtf, fabs(avisc_k ? hd / (r2 + 0.01 * hab * hab) : mu));
+                            const double mu = dot * rcp_pair(r2 + eta2 * hab * hab);
+                            const double alp = UH ? alp_k : alpha * hab;
+                            const double bet2 = UH ? bet2_k : 2.0 * beta * hab * hab;
+                            const double md =
+                                avisc_k ? dot * rcp_pair(r2 + 0.01 * hab * hab) : mu;
+                            dtf = fmax(dtf, mom_on ? fabs(UH ? md : md * hab) : 0.0);
                             // Monaghan Pi_ab when v_ab . r_ab < 0, selected, not branched on
-                            const double cab = 0.5 * (ca + r.c);
-                            const double rhoab = 0.5 * (rhoa + r.rho);
-                            const double piab = (-alpha * cab * mu + beta * mu * mu) / rhoab;
+                            const double c2 = ca + r.c, rho2 = rhoa + r.rho;
+                            const double piab = mu * fma(bet2, mu, -alp * c2) * rcp_pair(rho2);
                             tmp += dot < 0.0 ? piab : 0.0;
                         }
                         tmp *= -r.m;
-                        acc[0] += tmp * gx;
-                        acc[1] += tmp * gy;
-                        if (DIM == 3) acc[2] += tmp * gz;
+                        acc[0] += mom_on ? tmp * gx : 0.0;
+                        acc[1] += mom_on ? tmp * gy : 0.0;
+                        if (DIM == 3) acc[2] += mom_on ? tmp * gz : 0.0;
                     };
                 };
-                const int lc = list_count<LANES>(e, use_list, k, lane);
+                const int lc = list_count(e, use_list, k);
                 if (lc >= 0) {
                     auto from_list = [&](auto known) {
                         auto load = make_load(known);
-                        list_loop<LANES, FP64_BATCH>(
+                        auto use = make_use(known);
+                        list_loop<LANES, 2>(
                             e, k, lane, lc,
                             [&](uint32_t v) {
                                 int j;
                                 const bool ok = list_entry_d<DIM>(e, v, k, j);
                                 return load(j, ok);
                             },
-                            make_use(known));
+                            [&](const Rec &r, uint32_t) { use(r); });
                     };
                     switch (mode & 15) {   // block-uniform
                     case 0: from_list(std::integral_constant<int, 0>{}); break;
@@ -621,6 +625,7 @@ k_force(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask,
                 for (int d = 0; d < DIM; ++d) xs[d] += __shfl_xor_sync(0xffffffffu, xs[d], o);
             }
         }
+        dtf *= dt_h;
     }
 
     force_finish<DIM, F32, CONT>(e, cur, k, s, a, active, lane, acc, dtf, drho, xs,
@@ -632,20 +637,8 @@ static void launch_force_lr(const sphb_engine &e, int cur, uint32_t dm, int grav
                             bool cont, cudaStream_t st)
 {
     const dim3 g(e.num_pair_tiles), b(e.cfg.pair_block);
-    if (cont) {
-        launch_pdl(k_force<KT, DIM, F32, LV, RV, 4, true>, g, b, st, e, cur, dm, grav, mode);
-        return;
-    }
-    // the load-ahead depth only shapes the FP32C list loop of the cubic (the
-    // other kernels and FP64 load 4 ahead)
-    if constexpr (F32 && KT == SPHB_KERNEL_CUBIC) {
-        if (e.cfg.list_batch == 2) {
-            launch_pdl(k_force<KT, DIM, F32, LV, RV, 2, false>, g, b, st, e, cur, dm, grav,
-                       mode);
-            return;
-        }
-    }
-    launch_pdl(k_force<KT, DIM, F32, LV, RV, 4, false>, g, b, st, e, cur, dm, grav, mode);
+    if (cont) launch_pdl(k_force<KT, DIM, F32, LV, RV, true>, g, b, 0, st, e, cur, dm, grav, mode);
+    else launch_pdl(k_force<KT, DIM, F32, LV, RV, false>, g, b, 0, st, e, cur, dm, grav, mode);
 }
 
 template <int KT, int DIM, bool F32>

@@ -6,6 +6,10 @@
 //                           computed, one selected) for the list loops
 //   gw_bf(q, ir, ih, fac_ih) dW/dr / r in the reference's sign convention,
 //                           so grad_a W = (x_a - x_b) gw
+//   w_in, gw_in<CLAMP>      the same for the pair loops; without CLAMP inside
+//                           the support only.  gw_in keeps every factor of h
+//                           outside the polynomial: with one h in the scene
+//                           they are constants of the loop
 // with fac = norm<DIM>() / h^DIM, ih = 1 / h, ir = 1 / r, fac_ih = fac ih,
 // for T = float and double.  No form divides: the pair loops take one
 // reciprocal square root per pair and, with one h in the scene, the dest's
@@ -18,9 +22,55 @@
 
 namespace sphb {
 
+// Reciprocals and reciprocal square roots of the pair loops, without the
+// branches and the denormal scaling of the general forms (no pair's
+// denominators come near the denormals): a batch of pairs then is one
+// straight run of instructions, which the compiler interleaves.  FP32: the
+// hardware approximation.  FP64: the hardware's seed (relative error below
+// 2^-19), then one third-order step from the binomial series of 1 / (1 - e)
+// and 1 / sqrt(1 - e) in the seed's residual e; the results are within 2
+// units in the last place (tests/test_pair_math_gpu.py).
+__device__ __forceinline__ float rcp_pair(float x)
+{
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+__device__ __forceinline__ double rcp_pair(double x)
+{
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y, 1.0);
+    return fma(y, fma(e, e, e), y);
+}
+
+__device__ __forceinline__ float rsqrt_pair(float x)
+{
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+__device__ __forceinline__ double rsqrt_pair(double x)
+{
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double t = x * y, tl = fma(x, y, -t);   // x y exactly
+    const double e = fma(-tl, y, fma(-t, y, 1.0));
+    return fma(y, e * fma(0.375, e, 0.5), y);
+}
+
+// A product that no later sum contracts into an FMA.  The FP32C pair loops
+// write every product and FMA out this way: a loop in which h is a constant
+// and one in which it is the pair's then round alike, whatever the compiler
+// would contract in each.
+__device__ __forceinline__ float mul_pair(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_pair(double a, double b) { return __dmul_rn(a, b); }
+
 // 1 / r from r^2; finite at r = 0, where r^2 times it is 0.
-__device__ __forceinline__ float inv_dist(float r2) { return rsqrtf(fmaxf(r2, 1e-30f)); }
-__device__ __forceinline__ double inv_dist(double r2) { return rsqrt(fmax(r2, 1e-200)); }
+__device__ __forceinline__ float inv_dist(float r2) { return rsqrt_pair(fmaxf(r2, 1e-30f)); }
+__device__ __forceinline__ double inv_dist(double r2) { return rsqrt_pair(fmax(r2, 1e-200)); }
 
 template <int KT>
 struct Kern;
@@ -50,6 +100,24 @@ struct Kern<SPHB_KERNEL_CUBIC> {
         const T inner = (T(2.25) * q - T(3)) * ih;
         const T outer = T(-0.75) * t1 * t1 * ir;
         return fac_ih * (q < T(1) ? inner : outer);
+    }
+
+    template <bool CLAMP, typename T>
+    __device__ __forceinline__ static T w_in(T q, T fac)
+    {
+        const T t1 = CLAMP ? fmax(T(2) - q, T(0)) : T(2) - q;
+        const T inner = fma(q * q, fma(T(0.75), q, T(-1.5)), T(1));
+        const T outer = T(0.25) * t1 * (t1 * t1);
+        return fac * (q < T(1) ? inner : outer);
+    }
+
+    template <bool CLAMP, typename T>
+    __device__ __forceinline__ static T gw_in(T q, T ir, T ih, T fac_ih)
+    {
+        const T t1 = CLAMP ? fmax(T(2) - q, T(0)) : T(2) - q;
+        const T inner = fma(T(2.25) * (fac_ih * ih), q, T(-3) * (fac_ih * ih));
+        const T outer = (T(-0.75) * fac_ih) * ir * (t1 * t1);
+        return q < T(1) ? inner : outer;
     }
 };
 
@@ -89,6 +157,15 @@ struct Kern<SPHB_KERNEL_QUINTIC> {
         const T t1 = fmax(T(1) - q, T(0));
         return fac_ih * ir * fma(T(75), p4(t1), fma(T(-30), p4(t2), T(5) * p4(t3)));
     }
+
+    template <bool, typename T>
+    __device__ __forceinline__ static T w_in(T q, T fac) { return w_bf(q, fac); }
+
+    template <bool, typename T>
+    __device__ __forceinline__ static T gw_in(T q, T ir, T ih, T fac_ih)
+    {
+        return gw_bf(q, ir, ih, fac_ih);
+    }
 };
 
 // WendlandQuinticSplineKernel (S/base/kernels.pyx:562-640), 2D: support 2h,
@@ -116,6 +193,17 @@ struct Kern<SPHB_KERNEL_WENDLAND> {
     {
         const T t = fmax(fma(T(-0.5), q, T(1)), T(0));
         return fac_ih * ih * (T(-5) * (t * t * t));
+    }
+
+    template <bool, typename T>
+    __device__ __forceinline__ static T w_in(T q, T fac) { return w_bf(q, fac); }
+
+    template <bool CLAMP, typename T>
+    __device__ __forceinline__ static T gw_in(T q, T, T ih, T fac_ih)
+    {
+        T t = fma(T(-0.5), q, T(1));
+        if (CLAMP) t = fmax(t, T(0));
+        return (T(-5) * (fac_ih * ih)) * t * (t * t);
     }
 };
 

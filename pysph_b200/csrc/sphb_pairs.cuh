@@ -158,12 +158,15 @@ __device__ __forceinline__ uint32_t nbr_pack(int j, int o, int dy, int dz)
     return v;
 }
 
-// Each lane's list is padded with nbr_pad entries to a multiple of
-// SPHB_LIST_PAD slots, so the FP32 list loops load whole batches without a
-// per-entry bound.  A pad entry is the dest itself five cells away along x
-// (offset field 7): its squared distance exceeds every support radius
-// (cells are at least half the largest reach wide), so every pass rejects
-// it with the ordinary neighbour test.
+// A dest's list is one row of slots nbr[slot][k], entry s the s-th accepted
+// candidate whatever the number of threads that recorded it; LANES threads
+// read it in turn (thread l the slots l, l + LANES, ...), so their shares
+// differ by one entry at most.  It is padded with nbr_pad entries to a
+// multiple of SPHB_LIST_PAD slots a thread, so the list loops load whole
+// batches without a per-entry bound.  A pad entry is the dest itself five
+// cells away along x (offset field 7): its squared distance exceeds every
+// support radius (cells are at least half the largest reach wide), so every
+// pass rejects it with the ordinary neighbour test.
 constexpr int SPHB_LIST_PAD = 4;
 
 template <int DIM>
@@ -218,6 +221,12 @@ struct EntryF {
 };
 
 template <int DIM>
+__device__ __forceinline__ int entry_index(uint32_t v)
+{
+    return (int)(v & ((1u << (DIM == 2 ? SPHB_NBR_IDX_BITS_2D : SPHB_NBR_IDX_BITS_3D)) - 1u));
+}
+
+template <int DIM>
 __device__ __forceinline__ EntryF entry_unpack_f(uint32_t v)
 {
     constexpr int B = DIM == 2 ? SPHB_NBR_IDX_BITS_2D : SPHB_NBR_IDX_BITS_3D;
@@ -247,43 +256,174 @@ __device__ __forceinline__ bool list_entry_d(const sphb_engine &e, uint32_t v, i
     return ok;
 }
 
-// Entries of dest k this lane owns (-1 when some lane's list overflowed),
-// or -1 when the lists are not to be used.
-template <int LANES>
-__device__ __forceinline__ int list_count(const sphb_engine &e, bool use_list, int k, int lane)
+// Entries of dest k's list, or -1 when it overflowed or the lists are not
+// to be used.
+__device__ __forceinline__ int list_count(const sphb_engine &e, bool use_list, int k)
 {
-    if (!use_list) return -1;
-    const int N = e.cfg.num_particles;
-    int mine = 0;
-    bool ok = true;
-#pragma unroll
-    for (int l = 0; l < LANES; ++l) {
-        const int c = __ldg(e.f.nbr_cnt + (size_t)l * N + k);
-        ok = ok && c >= 0;
-        if (l == lane) mine = c;
-    }
-    return ok ? mine : -1;
+    return use_list ? __ldg(e.f.nbr_cnt + k) : -1;
 }
 
-// use(load(entry)) over the cnt list entries of (k, lane), in batches of
-// U: a batch's U neighbour records are loaded before any is used, and the
+// One dest's list being recorded by its LANES threads.
+template <int DIM, int LANES>
+struct ListWriter {
+    uint32_t *slots;    // nbr + k
+    size_t stride;      // slots are stride apart
+    int cap;            // slots that whole pads fill
+    int cnt;            // accepted so far, over the dest's threads
+    __device__ __forceinline__ ListWriter(uint32_t *nbr, int k, const sphb_engine &e)
+        : slots(nbr + k), stride(e.cfg.num_particles),
+          cap(e.f.list_cap - e.f.list_cap % (SPHB_LIST_PAD * LANES)), cnt(0)
+    {
+    }
+    // With LANES > 1 every thread of the warp calls it.
+    __device__ __forceinline__ void put(bool take, int j, int o, int dy, int dz)
+    {
+        int at = cnt;
+        if constexpr (LANES == 1) {
+            cnt += take;
+        } else {
+            const unsigned lane = threadIdx.x & (LANES - 1);
+            const unsigned in = (__ballot_sync(0xffffffffu, take) >> ((threadIdx.x & 31u) - lane)) &
+                                ((1u << LANES) - 1u);
+            at += __popc(in & ((1u << lane) - 1u));
+            cnt += __popc(in);
+        }
+        if (take && at < cap) slots[at * stride] = nbr_pack<DIM>(j, o, dy, dz);
+    }
+    // Pads after the last entry; the count, or -1 on overflow.
+    __device__ __forceinline__ int finish(int k)
+    {
+        if (cnt > cap) return -1;
+        constexpr int STEP = SPHB_LIST_PAD * LANES;
+        const int end = (cnt + STEP - 1) / STEP * STEP;
+        for (int c = cnt + (int)(threadIdx.x & (LANES - 1)); c < end; c += LANES)
+            slots[c * stride] = nbr_pad<DIM>(k);
+        return cnt;
+    }
+};
+
+// Shared memory of record_list for a block of `threads` threads.
+template <int DIM, int R, int LANES>
+constexpr int record_smem(int threads)
+{
+    return LANES > 1 ? (2 * R + 1) * (threads / LANES) * (int)sizeof(int2) : 0;
+}
+
+// Records dest k's list with LANES > 1 threads a dest: every candidate that
+// accept(j, o, dy, dz) takes, in the order of the full stencil.  Every thread
+// of the block calls it (active: k is a dest).  Returns the list's length, -1
+// when it overflowed.
+//
+// The row ranges of a stencil slab (2D: all rows; 3D: one z offset) go to
+// shared memory, and the threads take consecutive candidates of the rows as
+// of one run, so that every thread of the warp runs the longest of its
+// dests' runs and the accepted ones are numbered with one warp-wide ballot.
+// (A ballot over each dest's threads alone splits the warp: 45 -> 91 us, the
+// recording pass of an 86k-particle FP64 dam break with 2 threads a dest,
+// against 49 us this way.)
+template <int DIM, int R, int LANES, typename Accept>
+__device__ __forceinline__ int record_list(const sphb_engine &e, uint32_t *nbr, int2 *rows, int k,
+                                           bool active, uint32_t src_mask, int cell_base,
+                                           int ncells, const int *n, int local, int cx, int cy,
+                                           int cz, const CellTrim &trim, Accept &&accept)
+{
+    constexpr int NR = 2 * R + 1;
+    constexpr float RC2 = (R + 1e-3f) * (R + 1e-3f);
+    const int lane = threadIdx.x & (LANES - 1);
+    const int nd = blockDim.x / LANES;           // dests of the block
+    rows += threadIdx.x / LANES;
+    const int N = e.cfg.num_particles;
+    const int *__restrict__ start = e.work.start;
+    const int *__restrict__ cell = e.f.cell;
+    ListWriter<DIM, LANES> list(nbr, k, e);
+    if (active && !dest_cell_ok<DIM, R>(cx, cy, cz, n)) {
+        atomicOr(e.work.status, (unsigned)SPHB_ST_BAD_INDEX);
+        active = false;
+    }
+    for (int b = 0; b < e.cfg.num_arrays; ++b) {
+        if (!((src_mask >> b) & 1u)) continue;   // block-uniform
+        const int base = cell_base + b * ncells + local;
+#pragma unroll 1
+        for (int dz = (DIM == 3 ? -R : 0); dz <= (DIM == 3 ? R : 0); ++dz) {
+            // the slab's row ranges, empty for a row out of reach
+            __syncwarp();
+#pragma unroll 1
+            for (int i = lane; i < NR; i += LANES) {
+                const int dy = i - R;
+                int clo = -R, chi = R;   // x offsets of the cells to visit
+                if (DIM == 3 && trim.on) {
+                    const float ey = row_gap(trim.f[1], dy), ez = row_gap(trim.f[2], dz);
+                    const float ex = sqrtf(fmaxf(RC2 - ey * ey - ez * ez, 0.f));
+                    clo = max(-R, (int)floorf(trim.f[0] - ex));
+                    chi = min(R, (int)floorf(trim.f[0] + ex));
+                    if (RC2 - ey * ey - ez * ez < 0.f) chi = clo - 1;
+                }
+                int2 rg = make_int2(0, 0);
+                if (active && clo <= chi) {
+                    const int row = base + (dz * n[1] + dy) * n[0];
+                    rg = make_int2(__ldg(start + row + clo), __ldg(start + row + chi + 1));
+                    if (rg.x < 0 || rg.y > N || rg.x > rg.y) {
+                        atomicOr(e.work.status, (unsigned)SPHB_ST_BAD_INDEX);
+                        rg = make_int2(0, 0);
+                    }
+                }
+                rows[i * nd] = rg;
+            }
+            __syncwarp();
+            // (i, j): row and candidate, `skip` candidates on
+            int i = 0;
+            int2 rg = rows[0];
+            int j = rg.x;
+            auto advance = [&](int skip) {
+                j += skip;
+                while (j >= rg.y && ++i < NR) {
+                    j -= rg.y;
+                    rg = rows[i * nd];
+                    j += rg.x;
+                }
+            };
+            advance(lane);
+            while (__any_sync(0xffffffffu, i < NR)) {
+                bool take = false;
+                const int jc = j, dy = i - R;
+                int o = 0;
+                if (i < NR) {
+                    // the x offset from the candidate's own cell
+                    o = __ldg(cell + j) - (local + (dz * n[1] + dy) * n[0]);
+                    take = accept(j, o, dy, dz);
+                    advance(LANES);
+                }
+                list.put(take, jc, o, dy, dz);
+            }
+        }
+    }
+    int cnt = active ? list.finish(k) : -1;
+    __syncwarp();   // the list is read back by all its threads
+    return cnt;
+}
+
+// use(load(entry), entry) over this thread's share of the cnt entries of dest k's
+// list, in batches of U: a batch's U neighbour records are loaded before any is used, and the
 // next batch's list entries are fetched before this batch's records, so a
 // thread keeps U record gathers and U list loads in flight instead of one
-// dependent chain.  The last batch reads the list's pad entries (U divides
+// dependent chain.  (Loading a batch's records before the last batch is
+// used was slower at every register bound: 374 -> 409 us, the force pass of
+// 256 drops.)  The last batch reads the list's pad entries (U divides
 // SPHB_LIST_PAD), which the FP32C neighbour test rejects and the FP64 load
-// knows by their offset field (list_entry_d).
+// knows by their offset field (list_entry_d).  The entries are plain loads:
+// the density pass reads lists that it has just written.
 template <int LANES, int U, typename Load, typename Use>
 __device__ __forceinline__ void list_loop(const sphb_engine &e, int k, int lane, int cnt,
                                           Load &&load, Use &&use)
 {
     static_assert(SPHB_LIST_PAD % U == 0, "batches must end inside the padding");
     const int N = e.cfg.num_particles;
-    const uint32_t *__restrict__ p = e.f.nbr + (size_t)lane * N + k;
+    const uint32_t *p = e.f.nbr + (size_t)lane * N + k;
     const size_t stride = (size_t)LANES * N;
-    const int nb = (cnt + U - 1) / U;
+    const int nb = (cnt + U * LANES - 1) / (U * LANES);
     auto fetch = [&](int b, uint32_t *v) {
 #pragma unroll
-        for (int u = 0; u < U; ++u) v[u] = __ldg(p + (size_t)(b * U + u) * stride);
+        for (int u = 0; u < U; ++u) v[u] = p[(size_t)(b * U + u) * stride];
     };
     uint32_t v[U];
     if (nb > 0) fetch(0, v);
@@ -295,14 +435,14 @@ __device__ __forceinline__ void list_loop(const sphb_engine &e, int k, int lane,
 #pragma unroll
         for (int u = 0; u < U; ++u) r[u] = load(v[u]);
 #pragma unroll
-        for (int u = 0; u < U; ++u) use(r[u]);
+        for (int u = 0; u < U; ++u) use(r[u], v[u]);
 #pragma unroll
         for (int u = 0; u < U; ++u) v[u] = w[u];
     }
 }
 
 // The pairs of dest k: its list from the last density pass when use_list
-// and every lane's list is complete, else the cell search.
+// and it is complete, else the cell search.
 template <int DIM, int R, int LANES, typename F>
 __device__ __forceinline__ void traverse(const sphb_engine &e, bool use_list, int k, int lane,
                                          const int *__restrict__ start, int num_arrays,
@@ -311,25 +451,16 @@ __device__ __forceinline__ void traverse(const sphb_engine &e, bool use_list, in
                                          const CellTrim &trim, F &&f)
 {
     const int N = e.cfg.num_particles;
-    if (use_list) {
-        bool ok = true;
-        int mine = 0;
-#pragma unroll
-        for (int l = 0; l < LANES; ++l) {
-            const int c = __ldg(e.f.nbr_cnt + (size_t)l * N + k);
-            ok = ok && c >= 0;
-            if (l == lane) mine = c;
+    const int cnt = list_count(e, use_list, k);
+    if (cnt >= 0) {
+        const uint32_t *__restrict__ nbr = e.f.nbr;
+        for (int c = lane; c < cnt; c += LANES) {
+            int j, o, dy, dz;
+            nbr_unpack<DIM>(__ldg(nbr + (size_t)c * N + k), j, o, dy, dz);
+            if (j < N) f(j, o, dy, dz);
+            else atomicOr(e.work.status, (unsigned)SPHB_ST_BAD_INDEX);
         }
-        if (ok) {
-            const uint32_t *__restrict__ nbr = e.f.nbr;
-            for (int c = 0; c < mine; ++c) {
-                int j, o, dy, dz;
-                nbr_unpack<DIM>(__ldg(nbr + (size_t)(lane + LANES * c) * N + k), j, o, dy, dz);
-                if (j < N) f(j, o, dy, dz);
-                else atomicOr(e.work.status, (unsigned)SPHB_ST_BAD_INDEX);
-            }
-            return;
-        }
+        return;
     }
     for_each_candidate<DIM, R, LANES>(start, num_arrays, src_mask, cell_base, ncells, n, cx, cy,
                                       cz, lane, N, e.work.status, trim, f);
