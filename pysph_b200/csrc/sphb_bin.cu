@@ -57,7 +57,6 @@ __device__ __forceinline__ void grid_barrier(const sphb_engine &e, int *word_)
                 flag(e, SPHB_ST_STAGE_TIMEOUT);
                 break;
             }
-            __nanosleep(32);
         }
         __threadfence();
     }
@@ -221,81 +220,131 @@ k_refresh(const __grid_constant__ sphb_engine e, int cur)
     if (e.f.anchor) warp_max_disp(e, s, d2);
 }
 
-// ----------------------------------------------------------- grid setup --
-// Block 0 (<= 1024 threads).  Grid of scene s: cells floor(lo/cs)-R .. floor(hi/cs)+R per
-// axis (R padding cells, so every stencil row of every particle exists);
-// exclusive prefix of A*ncells over scenes gives the scene key bases.
-__device__ void grid_setup_block(const sphb_engine &e)
+// ------------------------------------------------- box accumulators --
+// The rebin's own box of scene s: six order-encoded maxima, of -x, -y, -z and
+// x, y, z, in the workspace behind the barrier's words.  Zero, below every
+// encoded double, is empty; block 0 clears them once every block has read
+// them, so no launch needs a phase that resets them.
+__device__ __forceinline__ unsigned long long *box_acc(const sphb_engine &e, int s)
 {
-    __shared__ long long sh[1024];
-    __shared__ long long s_carry;
-    const int S = e.cfg.num_scenes, A = e.cfg.num_arrays, R = e.cfg.stencil;
-    const int dim = e.cfg.dim;
+    const size_t nb = (size_t)(e.cfg.cell_capacity + SPHB_SCAN_CHUNK - 1) / SPHB_SCAN_CHUNK;
+    const size_t words = (nb + 1 + 64 + 1) & ~(size_t)1;   // 8-byte aligned
+    return (unsigned long long *)(e.work.bsum + words) + 6 * (size_t)s;
+}
+
+// ----------------------------------------------------------- grid setup --
+// Grid of scene s from its box: cells floor(lo/cs)-R .. floor(hi/cs)+R per
+// axis (R padding cells, so every stencil row of every particle exists).
+// Returns the cells of all its arrays, 0 (and a one-cell grid) when the box
+// does not fit the capacity.
+struct SceneGrid {
+    int lo[3], n[3];
+    int base, ncells;   // first key, cells per array
+};
+
+__device__ __forceinline__ long long scene_grid(const sphb_engine &e, int s, SceneGrid &g,
+                                                bool &bad)
+{
+    const unsigned long long *acc = box_acc(e, s);
+    const double cs = e.scene[s].cell_size;
+    const int R = e.cfg.stencil;
+    bad = false;
+    for (int d = 0; d < 3; ++d) {
+        g.lo[d] = 0;
+        g.n[d] = 1;
+    }
+    for (int d = 0; d < e.cfg.dim; ++d) {
+        const unsigned long long el = acc[d], eh = acc[3 + d];
+        double blo = -dec_double(el), bhi = dec_double(eh);
+        if (el == 0ull || eh == 0ull || !(blo <= bhi)) { blo = 0.0; bhi = 0.0; }
+        const double flo = floor(blo / cs), fhi = floor(bhi / cs);
+        if (!(fabs(flo) < 1.0e9) || !(fabs(fhi) < 1.0e9) || !(fhi - flo < 1.0e8)) {
+            bad = true;
+        } else {
+            g.lo[d] = (int)flo - R;
+            g.n[d] = (int)(fhi - flo) + 1 + 2 * R;
+        }
+    }
+    const long long need = (long long)e.cfg.num_arrays * g.n[0] * g.n[1] * g.n[2];
+    if (bad || need > e.cfg.cell_capacity) bad = true;
+    return bad ? 0 : need;
+}
+
+// The grids of all scenes, key bases by an exclusive prefix over the scenes'
+// cells; every thread of the block calls it.  grid != NULL (num_scenes <=
+// blockDim): the grids go to this shared array.  publish (one block): they
+// go to the scene states, with the boxes and the rebin's marks.  Returns the
+// cells in use.
+__device__ long long grids_setup(const sphb_engine &e, SceneGrid *grid, bool publish)
+{
+    __shared__ long long sh[SPHB_ELEM_TILE];
+    const int S = e.cfg.num_scenes, A = e.cfg.num_arrays;
     const long long cap = e.cfg.cell_capacity;
-    if (threadIdx.x == 0) s_carry = 0;
-    __syncthreads();
+    long long carry = 0;
     for (int base = 0; base < S; base += blockDim.x) {
         const int s = base + threadIdx.x;
-        long long need = 0;
-        int lo[3] = {0, 0, 0}, n[3] = {1, 1, 1};
+        SceneGrid g;
         bool bad = false;
-        if (s < S) {
-            const sphb_scene &sc = e.scene[s];
-            sphb_scene_state &st = e.sstate[s];
-            const double cs = sc.cell_size;
-            for (int d = 0; d < dim; ++d) {
-                double blo = dec_double(st.box[d]);
-                double bhi = dec_double(st.box[3 + d]);
-                if (!(blo <= bhi)) { blo = 0.0; bhi = 0.0; }
-                const double flo = floor(blo / cs), fhi = floor(bhi / cs);
-                if (!(fabs(flo) < 1.0e9) || !(fabs(fhi) < 1.0e9) ||
-                    !(fhi - flo < 1.0e8)) {
-                    bad = true;
-                    lo[d] = 0;
-                    n[d] = 1;
-                } else {
-                    lo[d] = (int)flo - R;
-                    n[d] = (int)(fhi - flo) + 1 + 2 * R;
-                }
-            }
-            need = (long long)A * n[0] * n[1] * n[2];
-            if (bad || need > cap) { bad = true; need = 0; }
-        }
-        sh[threadIdx.x] = need;
+        const long long need = s < S ? scene_grid(e, s, g, bad) : 0;
+        long long incl = need;
         __syncthreads();
-        for (int off = 1; off < (int)blockDim.x; off <<= 1) {
-            long long v = (int)threadIdx.x >= off ? sh[threadIdx.x - off] : 0;
+        if (S > 1) {   // inclusive prefix over the block
+            const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const long long v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += v;
+            }
+            if (lane == 31) sh[w] = incl;
             __syncthreads();
-            sh[threadIdx.x] += v;
-            __syncthreads();
+            long long before = 0, total = 0;
+            for (int i = 0; i < (int)(blockDim.x >> 5); ++i) {
+                if (i < w) before += sh[i];
+                total += sh[i];
+            }
+            incl += before;
+            sh[32 + 0] = total;   // (the same value from every thread)
+        } else if (threadIdx.x == 0) {
+            sh[32] = need;
         }
-        const long long incl = sh[threadIdx.x];
-        const long long total = sh[blockDim.x - 1];
+        __syncthreads();
+        const long long total = sh[32];
         if (s < S) {
-            sphb_scene_state &st = e.sstate[s];
-            const long long cb = s_carry + incl - need;
+            const long long cb = carry + incl - need;
             if (bad || cb + need > cap) {
-                flag(e, SPHB_ST_GRID_OVERFLOW);
-                for (int d = 0; d < 3; ++d) { st.lo[d] = 0; st.n[d] = 1; }
-                st.cell_base = 0;
-                st.ncells = 0;
+                if (publish) flag(e, SPHB_ST_GRID_OVERFLOW);
+                for (int d = 0; d < 3; ++d) { g.lo[d] = 0; g.n[d] = 1; }
+                g.base = 0;
+                g.ncells = 0;
             } else {
-                for (int d = 0; d < 3; ++d) { st.lo[d] = lo[d]; st.n[d] = n[d]; }
-                st.cell_base = (int)cb;
-                st.ncells = n[0] * n[1] * n[2];
+                g.base = (int)cb;
+                g.ncells = g.n[0] * g.n[1] * g.n[2];
             }
-            st.max_disp2 = 0ull;   // the anchors are the new positions
+            if (grid) grid[s] = g;
+            if (publish) {
+                sphb_scene_state &st = e.sstate[s];
+                const unsigned long long *acc = box_acc(e, s);
+                for (int d = 0; d < 3; ++d) {
+                    st.lo[d] = g.lo[d];
+                    st.n[d] = g.n[d];
+                    const unsigned long long el = acc[d], eh = acc[3 + d];
+                    st.box[d] = enc_double(el ? -dec_double(el) : INFINITY);
+                    st.box[3 + d] = enc_double(eh ? dec_double(eh) : -INFINITY);
+                }
+                st.cell_base = g.base;
+                st.ncells = g.ncells;
+                st.max_disp2 = 0ull;   // the anchors are the new positions
+            }
         }
-        __syncthreads();
-        if (threadIdx.x == 0) s_carry += total;
+        carry += total;
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        long long used = s_carry;
-        if (used > cap) {
-            flag(e, SPHB_ST_GRID_OVERFLOW);
-            used = 0;
-        }
+    long long used = carry;
+    if (used > cap) {
+        if (publish && threadIdx.x == 0) flag(e, SPHB_ST_GRID_OVERFLOW);
+        used = 0;
+    }
+    if (publish && threadIdx.x == 0) {
         e.work.meta[0] = (int)used;
         // new order: the lists must be recorded again before they are
         // reused; the positions are the anchors
@@ -307,6 +356,8 @@ __device__ void grid_setup_block(const sphb_engine &e)
         e.work.meta[4] = e.cfg.pair_mode == SPHB_PAIRS_TILED ? 1 : 0;
         e.work.meta[5] = 0;
     }
+    __syncthreads();
+    return used;
 }
 
 // ------------------------------------------------------- block work runs --
@@ -377,8 +428,8 @@ __device__ __forceinline__ void box_flush(const sphb_engine &e, int s, int dim, 
         double v = sh[0][c];
         for (int i = 1; i < (int)(blockDim.x >> 5); ++i)
             v = is_lo ? fmin(v, sh[i][c]) : fmax(v, sh[i][c]);
-        if (is_lo && v < INFINITY) atomicMin(&e.sstate[s].box[c], enc_double(v));
-        if (!is_lo && v > -INFINITY) atomicMax(&e.sstate[s].box[c], enc_double(v));
+        if (is_lo && v < INFINITY) atomicMax(&box_acc(e, s)[c], enc_double(-v));
+        if (!is_lo && v > -INFINITY) atomicMax(&box_acc(e, s)[c], enc_double(v));
     }
     __syncthreads();
 #pragma unroll
@@ -438,12 +489,21 @@ __device__ void box_accum_run(const sphb_engine &e, int cur, int t0, int t1)
 // Global cell key of a particle of segment seg at (x, y, z), or -1 (status
 // flagged) for a non-finite position or one outside its scene's grid.
 template <int DIM>
-__device__ __forceinline__ long long cell_key(const sphb_engine &e, int seg, double x, double y,
+__device__ __forceinline__ long long cell_key(const sphb_engine &e, const SceneGrid *grid,
+                                              long long used, int seg, double x, double y,
                                               double z)
 {
     const int A = e.cfg.num_arrays;
     const int s = seg / A, a = seg - s * A;
-    const sphb_scene_state &st = e.sstate[s];
+    SceneGrid st;
+    if (grid) {
+        st = grid[s];
+    } else {
+        const sphb_scene_state &q = e.sstate[s];
+        for (int d = 0; d < 3; ++d) { st.lo[d] = q.lo[d]; st.n[d] = q.n[d]; }
+        st.base = q.cell_base;
+        st.ncells = q.ncells;
+    }
     const double cs = e.scene[s].cell_size;
     const double p[3] = {x, y, z};
     int c[3] = {0, 0, 0};
@@ -462,18 +522,21 @@ __device__ __forceinline__ long long cell_key(const sphb_engine &e, int seg, dou
         c[d] = (int)f;
     }
     const int local = (c[2] * st.n[1] + c[1]) * st.n[0] + c[0];
-    const long long key = (long long)st.cell_base + (long long)a * st.ncells + local;
-    if (local >= st.ncells || key >= (long long)e.work.meta[0]) {
+    const long long key = (long long)st.base + (long long)a * st.ncells + local;
+    if (local >= st.ncells || key >= used) {
         flag(e, SPHB_ST_OUT_OF_GRID);
         return -1;
     }
     return key;
 }
 
-// Keys and the cell histogram: RU positions loaded, RU keys, RU atomics in
-// flight, then the stores.
+// Keys and the cell histogram: RU8 positions loaded, RU8 keys, RU8 atomics
+// in flight, then the stores.  totals: the scan chunks' totals too; a warp's
+// particles, sorted by cell since the last rebin, fall into one or two
+// chunks, with one atomic for each.
 template <int DIM>
-__device__ void hash_run(const sphb_engine &e, int cur, int t0, int t1)
+__device__ void hash_run(const sphb_engine &e, const SceneGrid *grid, long long used, int cur,
+                         int t0, int t1, bool totals)
 {
     const sphb_buffers &B = e.buf[cur];
     for (int t = t0; t < t1; t += RU8) {
@@ -492,7 +555,16 @@ __device__ void hash_run(const sphb_engine &e, int cur, int t0, int t1)
         long long key[RU8];
 #pragma unroll
         for (int u = 0; u < RU8; ++u)
-            key[u] = kk[u] >= 0 ? cell_key<DIM>(e, seg[u], px[u], py[u], pz[u]) : -1;
+            key[u] = kk[u] >= 0 ? cell_key<DIM>(e, grid, used, seg[u], px[u], py[u], pz[u]) : -1;
+        if (totals) {   // uniform over the launch
+#pragma unroll
+            for (int u = 0; u < RU8; ++u) {
+                const int chunk = key[u] >= 0 ? (int)(key[u] / SPHB_SCAN_CHUNK) : -1;
+                const unsigned same = __match_any_sync(0xffffffffu, chunk);
+                if (chunk >= 0 && (threadIdx.x & 31) == __ffs(same) - 1)
+                    atomicAdd(&e.work.bsum[chunk], __popc(same));
+            }
+        }
         int slot[RU8];
 #pragma unroll
         for (int u = 0; u < RU8; ++u) slot[u] = key[u] >= 0 ? atomicAdd(&e.work.count[key[u]], 1) : 0;
@@ -575,8 +647,9 @@ __device__ __forceinline__ void scan_reduce_chunk(const sphb_engine &e, int b, l
 
 // Chunk b: start[c] for its cells, start[T] after the last, and the counts
 // cleared for the next bin.  The chunk's offset is the sum of the totals
-// of the chunks before it, which every block adds up itself (a few
-// thousand L2-resident words at most), so no phase scans the totals.
+// of the chunks before it, which every block sums
+// itself (a few thousand L2-resident words at most), so no phase scans the
+// totals.
 __device__ __forceinline__ void scan_apply_chunk(const sphb_engine &e, int b, long long T,
                                                  bool vec)
 {
@@ -891,64 +964,87 @@ __device__ void copy_back_run(const sphb_engine &e, int cur, int mi, int t0, int
 }
 
 // ---------------------------------------------------------- the rebin --
-// One cooperative launch: [decision] -> boxes -> grids -> hash -> scan ->
-// scatter -> gather [-> copy back], the phases separated by grid_barrier.
-// With SPHB_BIN_IF_NEEDED block 0 decides first and every block returns
+// One cooperative launch, its phases separated by grid_barrier:
+//   [decision] and boxes | grids, keys, histogram, chunk totals | scan |
+//   scatter | gather [| copy back]
+// With SPHB_BIN_IF_NEEDED every block takes the decision first and returns
 // when the cells are kept; the gathered state then goes back to buf[cur].
+//
+// A rebin of few particles is a chain of latencies, above all the barriers
+// (~2.5 us each with 296 blocks): resetting the boxes, the decision's
+// commit, the grids and the chunk totals used to be phases of their own (ten
+// barriers).  The accumulators of the box and the totals are now left clear
+// by the rebin before, the commit waits for the first barrier, and every
+// block sets up the grids for itself (more than 256 scenes: block 0 alone,
+// one more barrier): a full
+// rebin 35 -> 27 us at 5k particles, 38 -> 31 us at 60k, 85 -> 81 us at 332k, 296 -> 285 us for
+// 256 drops (2.9M).
 template <int DIM, bool F32>
 __global__ void __launch_bounds__(SPHB_ELEM_TILE)
 k_rebin(const __grid_constant__ sphb_engine e, int cur, int flags)
 {
+    __shared__ SceneGrid s_grid[SPHB_ELEM_TILE];
     const bool if_needed = (flags & SPHB_BIN_IF_NEEDED) != 0;
     const int mi = (flags & SPHB_BIN_MOVE_INITIAL) ? 1 : 0;
-    const int nt = e.num_tiles;
+    const int nt = e.num_tiles, S = e.cfg.num_scenes;
     const int nb = (int)((e.cfg.cell_capacity + SPHB_SCAN_CHUNK - 1) / SPHB_SCAN_CHUNK);
     int *const bar = e.work.bsum + nb + 1;   // the barrier's word
     const int step_begin = (flags & SPHB_BIN_STEP_BEGIN) ? 1 : 0;
-    if (if_needed) {
-        bool lists;
-        if (decide_keep(e, &lists)) {   // block-uniform, the same in every block
-            // kept: the last block to arrive (every block has read the
-            // inputs by then) commits; nobody waits
-            __shared__ int s_last;
-            if (threadIdx.x == 0) {
-                __threadfence();
-                int *arrive = bar + 1;
-                s_last = atomicAdd(arrive, 1) == (int)gridDim.x - 1;
-                if (s_last) *arrive = 0;
-            }
-            __syncthreads();
-            if (s_last) decide_commit(e, step_begin, true, lists);
-            pdl_trigger();   // the density pass may launch
-            return;
+    bool lists = false;
+    if (if_needed && decide_keep(e, &lists)) {   // block-uniform, the same in every block
+        // kept: the last block to arrive (every block has read the
+        // inputs by then) commits; nobody waits
+        __shared__ int s_last;
+        if (threadIdx.x == 0) {
+            __threadfence();
+            int *arrive = bar + 1;
+            s_last = atomicAdd(arrive, 1) == (int)gridDim.x - 1;
+            if (s_last) *arrive = 0;
         }
-        grid_barrier(e, bar);   // every block has read the inputs
-        if (blockIdx.x == 0) decide_commit(e, step_begin, false, lists);
+        __syncthreads();
+        if (s_last) decide_commit(e, step_begin, true, lists);
+        pdl_trigger();   // the density pass may launch
+        return;
     }
-    // every rebin measures the scene boxes afresh (only a rebin reads them)
-    if (blockIdx.x == 0)
-        for (int s = threadIdx.x; s < e.cfg.num_scenes; s += blockDim.x) box_reset_scene(e, s);
-    grid_barrier(e, bar);
+    // every rebin measures the scene boxes afresh
     int t0, t1;
     block_tile_run(nt, t0, t1);
     box_accum_run<DIM>(e, cur, t0, t1);
+    grid_barrier(e, bar);   // every block has read the decision's inputs
+    if (if_needed && blockIdx.x == 0) decide_commit(e, step_begin, false, lists);
+    long long T;   // cells in use
+    const SceneGrid *grid = nullptr;
+    if (S <= (int)blockDim.x) {
+        T = grids_setup(e, s_grid, blockIdx.x == 0);
+        grid = s_grid;
+    } else {
+        if (blockIdx.x == 0) grids_setup(e, nullptr, true);
+        grid_barrier(e, bar);
+        T = *(volatile int *)&e.work.meta[0];
+    }
+    // few particles: the chunk totals with the histogram (an atomic per warp)
+    // instead of a pass over the counts and its barrier; many: the pass is
+    // the shorter one (2.9M particles: rebin 285 us against 314)
+    const bool totals = nt <= 2 * (int)gridDim.x;
+    hash_run<DIM>(e, grid, T, cur, t0, t1, totals);
     grid_barrier(e, bar);
-    if (blockIdx.x == 0) grid_setup_block(e);
-    grid_barrier(e, bar);
-    hash_run<DIM>(e, cur, t0, t1);
-    grid_barrier(e, bar);
+    if (blockIdx.x == 0)   // read by every block before this barrier
+        for (int i = threadIdx.x; i < 6 * S; i += blockDim.x) box_acc(e, 0)[i] = 0ull;
     // the scan covers the cells the grids use, not the whole capacity
-    const long long T = *(volatile int *)&e.work.meta[0];
     const int nbu = (int)((T + SPHB_SCAN_CHUNK - 1) / SPHB_SCAN_CHUNK);
     const bool vec = ((reinterpret_cast<uintptr_t>(e.work.count) |
                        reinterpret_cast<uintptr_t>(e.work.start)) & 15) == 0;
-    for (int b = blockIdx.x; b < nbu; b += gridDim.x) scan_reduce_chunk(e, b, T, vec);
-    grid_barrier(e, bar);
+    if (!totals) {
+        for (int b = blockIdx.x; b < nbu; b += gridDim.x) scan_reduce_chunk(e, b, T, vec);
+        grid_barrier(e, bar);
+    }
     if (T == 0) {
         if (blockIdx.x == 0 && threadIdx.x == 0) e.work.start[0] = 0;
     }
     for (int b = blockIdx.x; b < nbu; b += gridDim.x) scan_apply_chunk(e, b, T, vec);
     grid_barrier(e, bar);
+    if (blockIdx.x == gridDim.x - 1)   // summed by every block before this barrier
+        for (int i = threadIdx.x; i < nbu; i += blockDim.x) e.work.bsum[i] = 0;
     scatter_run(e, t0, t1);
     grid_barrier(e, bar);
     reorder_run<DIM, F32>(e, cur, mi, t0, t1);
@@ -1045,13 +1141,9 @@ static int rebin_grid(int *out)
     return SPHB_OK;
 }
 
-// Blocks of a launch: about 4 tiles each, between 2 per SM (a kept-cells
-// launch costs little more than one small kernel) and every resident block
-// (2 per SM at the rebin's 128 registers).  Measured on B200 with the
-// 332k-particle dam break: a kept-cells launch 4.6 us in a graph (a
-// one-block kernel 3.1 us), a full rebin 86-92 us; 256 drops (2.9M
-// particles) 375 us, of which the gather and the copy back, near the HBM
-// rate, are 260 us.
+// Blocks of a launch: one per tile up to 2 per SM (every resident block, at
+// the rebin's 128 registers), so that a small engine's barriers and
+// decisions wait for its own blocks only.
 template <int DIM, bool F32>
 static int launch_rebin_t(const sphb_engine *e, int cur, int flags, cudaStream_t st)
 {
@@ -1061,9 +1153,10 @@ static int launch_rebin_t(const sphb_engine *e, int cur, int flags, cudaStream_t
     cudaGetDevice(&dev);
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
         sms = 1;
-    int blocks = (e->num_tiles + 3) / 4;
-    if (blocks < 2 * sms) blocks = 2 * sms;
+    int blocks = e->num_tiles;
+    if (blocks > 2 * sms) blocks = (blocks + 3) / 4 > 2 * sms ? (blocks + 3) / 4 : 2 * sms;
     if (blocks > resident) blocks = resident;
+    if (blocks < 1) blocks = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(SPHB_ELEM_TILE);
