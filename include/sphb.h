@@ -227,6 +227,11 @@ typedef struct {
      * here, so the caller swaps geo <-> geo_next and vel <-> vel_next after
      * it.  When set, the rebin and sphb_refresh write both copies. */
     void *geo_next, *vel_next;
+    /* Optional (FP64): the second copy of the state's positions and
+     * velocities for the same stage: the pass reads buf[cur].x .. w and writes
+     * the moved particles' new ones here, so the caller swaps the two after
+     * it.  When set, the rebin and the imports write both copies. */
+    double *x_next, *y_next, *z_next, *u_next, *v_next, *w_next;
     int32_t list_cap;       /* slots per particle, 0 = no lists */
     int32_t pad0;
 } sphb_fields;
@@ -416,10 +421,11 @@ SPHB_API int sphb_tait(const sphb_engine *e, int cur, uint32_t dest_mask, void *
 /* mode | SPHB_FORCE_NO_MAXIMA: leave the per-scene dt_fac / |a| maxima
  * alone (a predictor's pass, whose maxima the CFL rule does not read). */
 #define SPHB_FORCE_NO_MAXIMA 32
-/* mode | SPHB_FORCE_STAGE(kind), FP32C with f.geo_next / vel_next: the
- * sphb_pc_stage stage `kind` (0..7) of every dest particle in the pass's
- * epilogue, on the accelerations, density rate and XSPH velocity it has
- * just computed.  The new records go to geo_next / vel_next; every stepped
+/* mode | SPHB_FORCE_STAGE(kind), FP32C with f.geo_next / vel_next, FP64 with
+ * f.x_next .. w_next: the sphb_pc_stage stage `kind` (0..7) of every dest
+ * particle in the pass's epilogue, on the accelerations, density rate and
+ * XSPH velocity it has just computed.  The new records (FP32C) or positions
+ * and velocities (FP64) go to the second copy; every stepped
  * array (cfg.step_on) and density-rate dest must be a dest of the pass.
  * Unlike sphb_pc_stage, stage 0 does not clear the CFL maxima: give the
  * predictor's pass (and RK2's first, RK4's first three)

@@ -107,7 +107,8 @@ class Buffers(ctypes.Structure):
 
 FIELD_NAMES = ("rho", "p", "cs", "au", "av", "aw", "dt_fac", "geo", "mass",
                "vel", "thermo", "cell", "nbr", "nbr_cnt", "anchor", "drho", "xu", "xv", "xw",
-               "geo_next", "vel_next")
+               "geo_next", "vel_next", "x_next", "y_next", "z_next", "u_next", "v_next",
+               "w_next")
 FORCE_USE_LIST = 16
 # cfg.pair_mode: neighbour lists (0) or shared-memory tiles (1)
 PAIRS_LISTS, PAIRS_TILED = 0, 1

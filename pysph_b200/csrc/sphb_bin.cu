@@ -794,6 +794,22 @@ __device__ __forceinline__ void carried_store(const sphb_buffers &S, const sphb_
     }
 }
 
+// The second copy of the positions and velocities (engines whose FP64 force
+// pass runs the integrator stage; the pointers decide).
+template <int DIM>
+__device__ __forceinline__ void next_store(const sphb_engine &e, int k, const Carried<DIM> &c)
+{
+    if (!e.f.x_next) return;
+    e.f.x_next[k] = c.x;
+    e.f.y_next[k] = c.y;
+    e.f.u_next[k] = c.u;
+    e.f.v_next[k] = c.v;
+    if (DIM == 3) {
+        e.f.z_next[k] = c.z;
+        e.f.w_next[k] = c.w;
+    }
+}
+
 // RK4's running sums of particle p to position k (engines that step RK4
 // have them; the pointers decide, uniformly over the launch).
 template <int DIM>
@@ -892,6 +908,7 @@ __device__ void reorder_run(const sphb_engine &e, int cur, int mi, int t0, int t
                 const int u = u0 + j;
                 if (k[u] < 0) continue;
                 carried_store<DIM>(S, D, k[u], mi, c[j]);
+                if (!F32) next_store<DIM>(e, k[u], c[j]);
                 if (mi) carry_sums<DIM>(S, D, p[u], k[u]);
                 const int s = seg[u] / A, a = seg[u] - s * A;
                 const sphb_scene_state &st = e.sstate[s];

@@ -27,10 +27,16 @@ extern "C" int sphb_momentum(const sphb_engine *e, int cur, uint32_t dest_mask,
     if (kind > 7) return SPHB_ERR_ARG;
     if ((rc = check_stage_sums(e, cur, kind))) return rc;
     if (kind >= 0) {
-        // the fused stage: FP32C, both record copies, the stage buffers,
+        // the fused stage: both copies of what it moves, the stage buffers,
         // and every stepped / density-rate array a dest of this pass
         const sphb_config &c = e->cfg;
-        if (c.precision != SPHB_FP32C || !e->f.geo_next || !e->f.vel_next) return SPHB_ERR_ARG;
+        if (c.precision == SPHB_FP32C) {
+            if (!e->f.geo_next || !e->f.vel_next) return SPHB_ERR_ARG;
+        } else {
+            if (!e->f.x_next || !e->f.y_next || !e->f.u_next || !e->f.v_next ||
+                (c.dim == 3 && (!e->f.z_next || !e->f.w_next)))
+                return SPHB_ERR_ARG;
+        }
         const sphb_buffers &B = e->buf[cur];
         if (!B.x0 || !B.y0 || !B.u0 || !B.v0 || (c.dim == 3 && (!B.z0 || !B.w0)))
             return SPHB_ERR_ARG;

@@ -99,33 +99,37 @@ __device__ __forceinline__ void force_finish(const sphb_engine &e, int cur, int 
             atomic_max_nonneg(&sw.max_acc2, ba2);
         }
     }
-    if constexpr (F32) {
-        // the integrator stage fused into the epilogue (FP32C): the rates
-        // as stored above, the new records into the second copy
-        const int kind = ((mode & SPHB_FORCE_STAGE_MASK) >> 8) - 1;
-        if (kind >= 0) {
-            const bool stepped = (e.cfg.step_on >> a) & 1u;
-            float d2 = 0.f;
-            if (active && lane == 0 && (stepped || rm)) {
-                const bool real = e.buf[cur].tag[k] == 0;
-                double f[3], xv[3];
+    // the integrator stage fused into the epilogue: the rates as stored
+    // above, the new records (FP32C) or state (FP64) into the second copy.
+    // In FP64 it replaces a launch of 3.5 us (5k particles) to 5.9 us (86k)
+    // that re-reads the rates, for 1.5 to 2.3 us more of the pass: 5k drop 58.8
+    // -> 55.7 us per step, 86k dam break 123 -> 116 us
+    const int kind = ((mode & SPHB_FORCE_STAGE_MASK) >> 8) - 1;
+    if (kind >= 0) {
+        const bool stepped = (e.cfg.step_on >> a) & 1u;
+        float d2 = 0.f;
+        if (active && lane == 0 && (stepped || rm)) {
+            const bool real = e.buf[cur].tag[k] == 0;
+            auto stored = [](double v) { return F32 ? (double)(float)v : v; };
+            double f[3], xv[3];
 #pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    f[d] = (double)(float)acc[d];
-                    xv[d] = (double)(float)(real ? xs[d] : 0.0);
-                }
-                const double dr = (double)(float)(real ? drho : 0.0);
-                const float4 g_old = ((const float4 *)e.f.geo)[k];
-                d2 = stage_particle<DIM, true>(e, cur, k, s, a, kind, f, xm != 0u, xv, dr,
-                                               (float4 *)e.f.geo_next, e.f.vel_next, g_old);
+            for (int d = 0; d < 3; ++d) {
+                f[d] = stored(acc[d]);
+                xv[d] = stored(real ? xs[d] : 0.0);
             }
-            if (stepped && e.f.anchor) warp_max_disp(e, s, d2);
-            if (blockIdx.x == 0 && threadIdx.x == 0) {
-                // the particles move: the lists are not known to be complete
-                // until the next rebin decision, and they leave the anchors
-                e.work.meta[2] = 0;
-                e.work.meta[3] = 0;
-            }
+            const double dr = stored(real ? drho : 0.0);
+            const float4 g_old =
+                F32 ? ((const float4 *)e.f.geo)[k] : make_float4(0.f, 0.f, 0.f, 0.f);
+            d2 = stage_particle<DIM, F32>(e, cur, k, s, a, kind, f, xm != 0u, xv, dr,
+                                          F32 ? (float4 *)e.f.geo_next : nullptr,
+                                          F32 ? e.f.vel_next : nullptr, g_old, !F32);
+        }
+        if (stepped && e.f.anchor) warp_max_disp(e, s, d2);
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            // the particles move: the lists are not known to be complete
+            // until the next rebin decision, and they leave the anchors
+            e.work.meta[2] = 0;
+            e.work.meta[3] = 0;
         }
     }
     block_add_u64(&e.work.pairs[1], np);

@@ -30,14 +30,17 @@ __device__ __forceinline__ double axpy_rn(double x0, double a, double dt)
 // acceleration, xv the XSPH velocity (when xsph), dr the density rate (used
 // for density-rate dests).  Non-LocalReal particles get zero rates.  With
 // geo_out / vel_out (FP32C) the particle's new pair records are written
-// there: g_old is its current geo record (the h, m it keeps).  Returns the
+// there: g_old is its current geo record (the h, m it keeps).  to_next (FP64):
+// the new position and velocity go to f.x_next .. w_next, because other
+// blocks may still read the old ones.  Returns the
 // squared FP32 distance from its anchor (0 without anchors or when the
 // array is not stepped).
 template <int DIM, bool F32>
 __device__ __forceinline__ float stage_particle(const sphb_engine &e, int cur, int k, int s,
                                                 int a, int stage, const double *f, bool xsph,
                                                 const double *xv, double dr, float4 *geo_out,
-                                                void *vel_out, float4 g_old)
+                                                void *vel_out, float4 g_old,
+                                                bool to_next = false)
 {
     const sphb_buffers &B = e.buf[cur];
     const sphb_scene_state &st = e.sstate[s];
@@ -76,6 +79,8 @@ __device__ __forceinline__ float stage_particle(const sphb_engine &e, int cur, i
     double *V[3] = {B.u, B.v, B.w};
     double *X0[3] = {B.x0, B.y0, B.z0};
     double *V0[3] = {B.u0, B.v0, B.w0};
+    double *XN[3] = {e.f.x_next, e.f.y_next, e.f.z_next};
+    double *VN[3] = {e.f.u_next, e.f.v_next, e.f.w_next};
     double *KX[3] = {B.kx, B.ky, B.kz};
     double *KV[3] = {B.ku, B.kv, B.kw};
     const bool real = B.tag[k] == 0;
@@ -117,8 +122,8 @@ __device__ __forceinline__ float stage_particle(const sphb_engine &e, int cur, i
         }
         p[d] = advance(x[d], x0[d], fx, KX[d]);
         vn[d] = advance(v[d], v0[d], fd, KV[d]);
-        X[d][k] = p[d];
-        V[d][k] = vn[d];
+        (to_next ? XN[d] : X[d])[k] = p[d];
+        (to_next ? VN[d] : V[d])[k] = vn[d];
     }
     float d2 = 0.f;
     // FP32 pair records of the new state, relative to the particle's cell of

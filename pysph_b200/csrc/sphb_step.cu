@@ -155,8 +155,16 @@ __device__ __forceinline__ void exchange_field(const sphb_engine &e, int cur, in
 {
     if (field <= 13 || field == 21 || field == 22) {
         double *f = field_ptr<F32>(e, cur, field);
-        if (dir == 0) f[k] = user[ui];
-        else user[ui] = f[k];
+        if (dir == 0) {
+            f[k] = user[ui];
+            if (!F32 && field <= 5 && e.f.x_next) {   // both copies
+                double *n[6] = {e.f.x_next, e.f.y_next, e.f.z_next,
+                                e.f.u_next, e.f.v_next, e.f.w_next};
+                if (n[field]) n[field][k] = user[ui];
+            }
+        } else {
+            user[ui] = f[k];
+        }
         return;
     }
     if (field >= 23) {   // _a_rho_1, XSPH velocity: scatter only

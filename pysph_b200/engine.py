@@ -388,6 +388,13 @@ class Engine:
             f["geo"] = f["mass"] = f["vel"] = None
             f["thermo"] = torch.zeros(N, **f64)   # P / rho^2 for the force pass
             f["geo_next"] = f["vel_next"] = None
+        # FP64: the second copy of the positions and velocities, for the same
+        # (an engine that keeps its cells between stages; else every rebin
+        # would swap the state buffers under the copies)
+        for name in ("x", "y", "z", "u", "v", "w"):
+            second = (not self.f32 and self.fuse_stage and self.step_lists
+                      and self.scheme.step_on and (dim == 3 or name not in ("z", "w")))
+            f[name + "_next"] = torch.zeros(N, **f64) if second else None
         f["cell"] = torch.zeros(N, **i32)
         # outputs of SPHDensityRate (_a_rho_1) and XSPHCorrection (velocity):
         # the continuity scheme's, and any single calc's on this engine
@@ -732,8 +739,9 @@ class Engine:
     @property
     def fuses_stage(self) -> bool:
         """Whether the integrator stage runs in the force pass's epilogue
-        (FP32C, with every stepped and density-rate array a force dest)."""
-        if not (self.f32 and self.fuse_stage):
+        (every stepped and density-rate array a force dest; in FP64 with the
+        cells kept between stages)."""
+        if not self.fuse_stage or (not self.f32 and self.fields["x_next"] is None):
             return False
         dests = self.scheme.pair_dests if self.scheme.continuity else self.scheme.mom_dests
         need = sum(1 << a for a in self.scheme.step_on)
@@ -742,6 +750,13 @@ class Engine:
 
     def _swap_records(self):
         f = self.fields
+        if not self.f32:
+            b, db = self.bufs[self.cur], self.desc.buf[self.cur]
+            for c in ("x", "y", "u", "v") + (("z", "w") if self.dim == 3 else ()):
+                b[c], f[c + "_next"] = f[c + "_next"], b[c]
+                setattr(db, c, b[c].data_ptr())
+                setattr(self.desc.f, c + "_next", f[c + "_next"].data_ptr())
+            return
         f["geo"], f["geo_next"] = f["geo_next"], f["geo"]
         f["vel"], f["vel_next"] = f["vel_next"], f["vel"]
         for name in ("geo", "geo_next", "vel", "vel_next"):
