@@ -515,6 +515,12 @@ SPHB_API int sphb_init_index(const sphb_engine *e, int cur, void *stream);
 SPHB_API int sphb_permute(const sphb_engine *e, int cur, int array, int dir, double *user,
                           double *engine_buf, const int32_t *user_offset, void *stream);
 
+/* sphb_permute of count (1..SPHB_EXCHANGE_MAX) buffers of one array in one
+ * launch (users, engine_bufs: host arrays of device pointers). */
+SPHB_API int sphb_permute_many(const sphb_engine *e, int cur, int array, int dir, int32_t count,
+                               double *const *users, double *const *engine_bufs,
+                               const int32_t *user_offset, void *stream);
+
 /* ---- adjoint of the particle update ---------------------------------
  * The reference has no gradients; these are the reverse-mode kernels of the
  * differentiable rollout (FP64 engines only).  Vectors are SoA [dim][N] in

@@ -81,8 +81,12 @@ class Rollout:
     def get_state(self, eng=None):
         eng = eng or self.fwd
         px, pv = self._comps()
-        return {a: (torch.stack([eng.get(a, c) for c in px]),
-                    torch.stack([eng.get(a, c) for c in pv])) for a in self.moving}
+        out = {}
+        for a in self.moving:
+            s = torch.empty(2 * self.dim, eng.user_n[a], dtype=torch.float64, device=self.device)
+            eng.exchange_out_many(a, px + pv, list(s))
+            out[a] = (s[:self.dim], s[self.dim:])
+        return out
 
     def set_state(self, state, eng=None, rebin=True):
         """The state into an engine, rebinned there: every restart from the
@@ -93,10 +97,7 @@ class Rollout:
         eng = eng or self.fwd
         px, pv = self._comps()
         for a, (X, V) in state.items():
-            for d, c in enumerate(px):
-                eng.exchange_in(a, c, X[d])
-            for d, c in enumerate(pv):
-                eng.exchange_in(a, c, V[d])
+            eng.exchange_in_many(a, list(zip(px + pv, list(X) + list(V))))
         eng.invalidate_box()
         if rebin:
             eng.rebin_now()
@@ -170,9 +171,7 @@ class Rollout:
         S = self._scratch
         self._scratch_buf.zero_()
         for a, L in lam_F.items():
-            for d in range(dim):
-                eng.call("sphb_permute", eng.cur, a, 0, L[d].contiguous().data_ptr(),
-                         S["lam_a"][d].data_ptr(), eng.user_offset[a].data_ptr())
+            eng.permute_many(a, 0, list(L.contiguous()), list(S["lam_a"]))
         mom = self.scheme.mom_dests
         eng.call("sphb_force_vjp", eng.cur, mom, S["lam_a"].data_ptr(), S["lam_x"].data_ptr(),
                  S["lam_v"].data_ptr(), S["lam_rho"].data_ptr(), S["lam_p"].data_ptr(),
@@ -183,15 +182,9 @@ class Rollout:
                  S["lam_x"].data_ptr())
         out = {}
         for a in self.moving:
-            n = eng.user_n[a]
-            lX = torch.empty(dim, n, dtype=torch.float64, device=dev)
-            lV = torch.empty(dim, n, dtype=torch.float64, device=dev)
-            for d in range(dim):
-                eng.call("sphb_permute", eng.cur, a, 1, lX[d].data_ptr(),
-                         S["lam_x"][d].data_ptr(), eng.user_offset[a].data_ptr())
-                eng.call("sphb_permute", eng.cur, a, 1, lV[d].data_ptr(),
-                         S["lam_v"][d].data_ptr(), eng.user_offset[a].data_ptr())
-            out[a] = (lX, lV)
+            l = torch.empty(2 * dim, eng.user_n[a], dtype=torch.float64, device=dev)
+            eng.permute_many(a, 1, list(l), list(S["lam_x"]) + list(S["lam_v"]))
+            out[a] = (l[:dim], l[dim:])
         return out
 
     def step_adjoint(self, s0, sh, lam):

@@ -896,6 +896,35 @@ class Engine:
             self.call("sphb_exchange_many", self.cur, array, direction, len(part), fields,
                       users, self.user_offset[array].data_ptr())
 
+    def exchange_in_many(self, array: int, items):
+        """exchange_in of several (position or velocity name, tensor) of one
+        array, in one launch when every tensor can be read as it is (FP64,
+        contiguous, on the engine's device)."""
+        items = [(n, t) for n, t in items if t.numel() or self.user_n[array]]
+        for n, t in items:
+            if not (n in ("x", "y", "z", "u", "v", "w") and t.dtype == torch.float64
+                    and t.device == self.device and t.is_contiguous()
+                    and t.numel() == self.user_n[array]):
+                for m, s in items:
+                    self.exchange_in(array, m, s)
+                return
+        if items:
+            self._exchange_many(array, 0, items)
+            # as _exchange_in: the next bin recomputes the boxes and refreshes
+            # the records
+            self._box_valid = False
+            self._host_state = True
+
+    def permute_many(self, array: int, direction: int, users, bufs):
+        """sphb_permute of several user-order tensors to (0) or from (1) engine
+        -order ones, EXCHANGE_MAX per launch."""
+        for i in range(0, len(users), nat.EXCHANGE_MAX):
+            u, b = users[i:i + nat.EXCHANGE_MAX], bufs[i:i + nat.EXCHANGE_MAX]
+            ptr = ctypes.c_void_p * len(u)
+            self.call("sphb_permute_many", self.cur, array, direction, len(u),
+                      ptr(*[t.data_ptr() for t in u]), ptr(*[t.data_ptr() for t in b]),
+                      self.user_offset[array].data_ptr())
+
     def exchange_out_many(self, array: int, names, outs):
         """exchange_out of several properties into the given FP64 tensors in
         one launch."""
