@@ -242,7 +242,7 @@ k_density(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask, in
                         };
                         w = hks ? 0.5f * (w_at(hk) + w_at(hj)) : w_at(0.5f * (hk + hj));
                     }
-                    acc.add(in ? mul_pair(r.m, w) : 0.f);
+                    acc.add_prod(r.m, w, in);
                     np += in;
                 };
                 // the common case (one h, every source summed, densities
@@ -261,7 +261,7 @@ k_density(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask, in
                     const bool in = r2 < rad2;
                     const float ir = inv_dist(r2);   // q = 0 at r = 0
                     const float w = Kern<KT>::template w_in<false>(mul_pair(r2 * ir, ihk), fack);
-                    acc.add(in ? mul_pair(r.m, w) : 0.f);
+                    acc.add_prod(r.m, w, in);
                     np += in;
                 };
                 if constexpr (LANES == 1) {

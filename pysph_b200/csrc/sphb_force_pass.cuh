@@ -344,12 +344,12 @@ k_force(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask,
                         }
                         if (CONT) {
                             // drho_a += m_b (v_a - v_b) . grad_a W
-                            kr.add(rate_on ? mul_pair(r.m, dot * gw) : 0.f);
+                            kr.add_prod(r.m, dot * gw, rate_on);
                             // XSPH: eps m_b W_ab (v_b - v_a) / rho_ab (eps at the end)
                             const float temp = r.m * w * rcp_pair(0.5f * (tk.x + r.t.x));
-                            kxx.add(xs_on ? mul_pair(-temp, vx) : 0.f);
-                            kxy.add(xs_on ? mul_pair(-temp, vy) : 0.f);
-                            if (DIM == 3) kxz.add(xs_on ? mul_pair(-temp, vz) : 0.f);
+                            kxx.add_prod(-temp, vx, xs_on);
+                            kxy.add_prod(-temp, vy, xs_on);
+                            if (DIM == 3) kxz.add_prod(-temp, vz, xs_on);
                         }
                         if (visc_k || avisc_k) {
                             // mu / h_ab = dot / (r^2 + eta^2 h_ab^2); the factors
@@ -373,9 +373,9 @@ k_force(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask,
                         // (the products are selected, so a NaN outside the
                         // support stays there)
                         const float f = -r.m * tmp * gw;
-                        ax.add(mom_on ? mul_pair(f, rx) : 0.f);
-                        ay.add(mom_on ? mul_pair(f, ry) : 0.f);
-                        if (DIM == 3) az.add(mom_on ? mul_pair(f, rz) : 0.f);
+                        ax.add_prod(f, rx, mom_on);
+                        ay.add_prod(f, ry, mom_on);
+                        if (DIM == 3) az.add_prod(f, rz, mom_on);
                     };
                 };
                 const int lc = list_count(e, use_list, k);

@@ -116,8 +116,7 @@ struct Kern<SPHB_KERNEL_CUBIC> {
     {
         const T t1 = CLAMP ? fmax(T(2) - q, T(0)) : T(2) - q;
         // (the polynomial's own constants stay exact: folding the factor into
-        // them too rounds each, and 2.25 q - 3 cancels; positions of a 20k
-        // drop after 40 FP32C steps were 11% further off)
+        // them too would round each, and 2.25 q - 3 cancels)
         const T inner = fma(T(2.25), q, T(-3)) * (fac_ih * ih);
         const T outer = (T(-0.75) * fac_ih) * ir * (t1 * t1);
         return q < T(1) ? inner : outer;
