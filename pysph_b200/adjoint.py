@@ -83,9 +83,13 @@ class Rollout:
         px, pv = self._comps()
         out = {}
         for a in self.moving:
-            s = torch.empty(2 * self.dim, eng.user_n[a], dtype=torch.float64, device=self.device)
-            eng.exchange_out_many(a, px + pv, list(s))
-            out[a] = (s[:self.dim], s[self.dim:])
+            # two tensors of their own, not views of one: a caller may modify
+            # or keep either (autograd refuses an in-place change of a view
+            # that a custom function returned)
+            X, V = (torch.empty(self.dim, eng.user_n[a], dtype=torch.float64,
+                                device=self.device) for _ in range(2))
+            eng.exchange_out_many(a, px + pv, list(X) + list(V))
+            out[a] = (X, V)
         return out
 
     def set_state(self, state, eng=None, rebin=True):
@@ -182,9 +186,10 @@ class Rollout:
                  S["lam_x"].data_ptr())
         out = {}
         for a in self.moving:
-            l = torch.empty(2 * dim, eng.user_n[a], dtype=torch.float64, device=dev)
-            eng.permute_many(a, 1, list(l), list(S["lam_x"]) + list(S["lam_v"]))
-            out[a] = (l[:dim], l[dim:])
+            lX, lV = (torch.empty(dim, eng.user_n[a], dtype=torch.float64, device=dev)
+                      for _ in range(2))
+            eng.permute_many(a, 1, list(lX) + list(lV), list(S["lam_x"]) + list(S["lam_v"]))
+            out[a] = (lX, lV)
         return out
 
     def step_adjoint(self, s0, sh, lam):
