@@ -768,9 +768,12 @@ class Engine:
         (the predictor's pass then leaves the CFL maxima alone), else as its
         own pass.  A fused stage swaps the two record copies, so a captured
         graph must hold an even number of them: a PC or RK2 step does, and
-        an Euler step (one stage) being captured runs its stage on its own."""
+        an Euler step (one stage) being captured runs its stage on its own.
+        In FP64 the copies are the state itself: a step must leave them where
+        it found them, or a graph that the caller captured before would go on
+        in the other one, so an FP64 Euler step never fuses its stage."""
         capturing = self.device.type == "cuda" and torch.cuda.is_current_stream_capturing()
-        if self.fuses_stage and not (kind == 2 and capturing):
+        if self.fuses_stage and not (kind == 2 and (capturing or not self.f32)):
             self.eval_stage(stage=kind)
             self._box_valid = True
         else:

@@ -61,6 +61,30 @@ def test_matches_the_separate_stage(name, integrator):
     same("host writes and graph replays")
 
 
+@pytest.mark.parametrize("integrator", ["pc", "euler", "rk2", "rk4"])
+def test_a_callers_graph_outlives_other_steps(integrator):
+    """A graph that a program captured itself holds the buffers' addresses, so
+    every step leaves the state where it found it: a captured PC step, then one
+    step of each integrator, then the graph again."""
+    arrays, params, scheme, dim = _case("dam")
+    engs = [Engine([(arrays, params)], scheme, dim=dim, precision="fp64", fuse_stage=f)
+            for f in (True, False)]
+    for e in engs:
+        for _ in range(2):
+            e.pc_step()
+        if integrator == "rk4":
+            e.step("rk4")       # makes its sums
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            e.pc_step()
+        g.replay()
+        e.step(integrator)
+        g.replay()
+        e.check_status()
+    for n in ("x", "y", "u", "v", "rho", "p"):
+        assert torch.equal(engs[0].get(0, n), engs[1].get(0, n)), n
+
+
 def test_needs_the_second_copy():
     arrays, params, scheme, dim = _case("dam")
     eng = Engine([(arrays, params)], scheme, dim=dim, precision="fp64", step_lists=False)
