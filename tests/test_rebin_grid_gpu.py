@@ -1,0 +1,55 @@
+"""The rebin's launch follows its work: particles and cells.  The number of
+blocks is read from a captured graph."""
+import numpy as np
+import pytest
+import torch
+from cuda.bindings import driver
+
+from pysph_b200 import _native as nat
+from pysph_b200.engine import Engine, fluid_scheme
+
+pytestmark = pytest.mark.gpu
+
+
+def _ok(res):
+    assert res[0] == driver.CUresult.CUDA_SUCCESS, res[0]
+    return res[1:]
+
+
+def _rebin_blocks(eng):
+    eng.rebin_now()
+    g = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(g):
+        eng.call("sphb_bin", eng.cur, nat.BIN_IF_NEEDED)
+    graph = driver.CUgraph(init_value=g.raw_cuda_graph())
+    _, n = _ok(driver.cuGraphGetNodes(graph, 0))
+    nodes, _ = _ok(driver.cuGraphGetNodes(graph, n))
+    return [_ok(driver.cuGraphKernelNodeGetParams(k))[0].gridDimX for k in nodes[:n]]
+
+
+def _engine(n, side, dim, **kw):
+    rng = np.random.default_rng(n)
+    x, y, z = rng.uniform(0, side, (3, n))
+    if dim == 2:
+        z = 0 * z
+    o = np.ones(n)
+    arr = dict(x=x, y=y, z=z, u=0 * o, v=0 * o, w=0 * o, m=o, h=0.4 * o, rho=o, p=0 * o, cs=o)
+    return Engine([([arr], dict(dt=1e-9))], fluid_scheme(1), dim=dim, precision="fp64", **kw)
+
+
+@pytest.mark.parametrize("dim,side", [(2, 1000.0), (3, 100.0)])
+def test_scattered_particles_get_the_blocks_their_cells_need(dim, side):
+    """1,000 particles (four tiles) over a million cells: the scan's 245
+    chunks are not left to four blocks."""
+    eng = _engine(1000, side, dim)
+    assert eng.cell_capacity > 1e6
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert _rebin_blocks(eng) == [2 * sms]
+    eng.check_status()
+
+
+@pytest.mark.parametrize("cells", [4096, 4097, 5 * 4096])
+def test_small_engines_wait_for_few_blocks(cells):
+    eng = _engine(1000, 10.0, 2, cell_capacity=cells)
+    assert _rebin_blocks(eng) == [max(4, -(-cells // 4096))]
+    eng.check_status()
