@@ -414,7 +414,11 @@ class Engine:
             # quintic): entries grow as (radius (1 + margin))^dim; a lane
             # whose list overflows searches its cells instead
             grow = ((1.0 + self.skin_margin) * nat.KERNEL_RADIUS[self.kernel] / 2.0) ** dim
-            self.list_cap = int(math.ceil(self.list_cap * grow / 8.0)) * 8
+            self.list_cap = int(math.ceil(self.list_cap * grow))
+            # whole batches of 4 entries for up to 8 threads a dest: a list
+            # fills pads of 4 x lanes slots, and no launch shape may round the
+            # capacity down
+            self.list_cap += -self.list_cap % 32
         if self.list_cap:
             f["nbr"] = torch.zeros(self.list_cap * N, **i32)
             f["nbr_cnt"] = torch.zeros(8 * N, **i32)

@@ -67,3 +67,36 @@ def test_lists_of_every_length(n, lanes, precision):
         again = eng.get(0, "rho").cpu().numpy()
         assert np.max(np.abs(again - O.rho) / O.rho) <= rtol
         eng.check_status()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32c"])
+@pytest.mark.parametrize("dim", [2, 3])
+def test_lists_as_long_as_the_capacity(dim, precision):
+    """Every slot of a list can hold an entry: a clump with as many particles
+    as there are slots keeps its lists, one more overflows them all (and the
+    passes search the cells).  The capacity covers h = 2 dx (66 entries in
+    2D with the skin)."""
+    params = dict(dim=dim, c0=10.0, rho0=100.0, gamma=1.0, alpha=0.1, beta=0.2, eta=0.1, dt=1e-5)
+    cap = Engine([([_cluster(1, dim, False)], params)], fluid_scheme(1), dim=dim,
+                 precision=precision).list_cap
+    assert cap >= (88 if dim == 2 else 248)
+    for n in (cap, cap + 1):
+        arr = _cluster(n, dim, False)
+        scheme = fluid_scheme(1)
+        eng = Engine([([arr], params)], scheme, dim=dim, precision=precision)
+        osys = oracle_from([arr], params, scheme, dim)
+        osys.update()
+        oracle_density_eos(osys, scheme)
+        O = osys.arrays[0]
+        eng.density()
+        rho = eng.get(0, "rho").cpu().numpy()
+        assert np.max(np.abs(rho - O.rho) / O.rho) <= TOL[precision][0]
+        assert bool((eng.fields["nbr_cnt"][:eng.N] == (n if n == cap else -1)).all())
+        listed = {}
+        for mode in (USE_LIST, 0):
+            eng.momentum(mode=mode)
+            listed[mode] = [eng.get(0, c).cpu().numpy() for c in ("au", "av", "aw")[:dim]]
+        scale = max(np.max(np.abs(s)) for s in listed[0])
+        for a, b in zip(listed[USE_LIST], listed[0]):
+            assert rel_err(a, b, scale) <= TOL[precision][1]
+        eng.check_status()
