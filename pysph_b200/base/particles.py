@@ -327,8 +327,8 @@ class Particles:
         self.kernel = None
         # launch shape of the engine behind these arrays (this build's own
         # option, no reference counterpart): Engine keyword arguments such
-        # as pairs, stencil, lanes, pair_block, skin_margin, e.g. from
-        # pysph_b200.autotune.autotune
+        # as pairs, stencil, lanes, exact_lanes, pair_block, skin_margin,
+        # e.g. from pysph_b200.autotune.autotune
         self.engine_options: dict = {}
         self.correction_manager = None
         self.misc_prop_update_functions = []

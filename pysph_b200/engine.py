@@ -157,7 +157,9 @@ class Engine:
 
     scenes: list of (arrays, params) where arrays is a list of dicts of
     numpy/torch FP64 properties (x, y, z, u, v, w, m, h, rho, p, cs, tag)
-    and params a SceneParams or dict."""
+    and params a SceneParams or dict.  lanes: threads per dest particle of
+    the pair passes, at least (lanes_for raises it for small engines); with
+    exact_lanes, exactly."""
 
     def __init__(self, scenes, scheme: Scheme, dim: int = 2,
                  precision: str = "fp32c", stencil: int = 1, lanes: int = 1,
@@ -166,7 +168,7 @@ class Engine:
                  step_lists: bool = True, skin_margin: float | None = None,
                  list_batch: int = 4, variable_h: bool = False,
                  kernel: int = nat.KERNEL_CUBIC, fuse_stage: bool = True,
-                 pairs: str = "lists"):
+                 pairs: str = "lists", exact_lanes: bool = False):
         if dim not in (2, 3):
             raise ValueError("dim must be 2 or 3")
         if precision not in ("fp64", "fp32c"):
@@ -262,6 +264,7 @@ class Engine:
         if list_batch not in (2, 4):
             raise ValueError("list_batch must be 2 or 4")
         self.list_batch = list_batch
+        self.exact_lanes = bool(exact_lanes)
         self._alloc(lanes, pair_block)
         self._upload(scenes)
 
@@ -441,7 +444,9 @@ class Engine:
         self.set_launch(lanes, pair_block)
 
     def _launch_lanes(self, lanes):
-        return lanes if self.pairs == "tiled" else lanes_for(self.N, lanes)
+        if self.exact_lanes or self.pairs == "tiled":
+            return lanes
+        return lanes_for(self.N, lanes)
 
     def _config(self, lanes, pair_block):
         cfg = nat.Config()
@@ -481,11 +486,14 @@ class Engine:
                   "sphb_make_tiles")
         return _struct_to_device(arr, self.device), n.value
 
-    def set_launch(self, lanes: int, pair_block: int, list_batch: int | None = None):
-        """Pair-kernel launch shape: lanes per dest particle (at least; see
-        lanes_for) and block size.  list_batch (2 or 4) is accepted as before:
-        the force pass loads two list entries ahead, which measured faster
-        than four on every workload."""
+    def set_launch(self, lanes: int, pair_block: int, list_batch: int | None = None,
+                   exact: bool | None = None):
+        """Pair-kernel launch shape: lanes per dest particle and block size.
+        The engine runs at least `lanes` (lanes_for) or, with exact, exactly
+        as many (None: as the engine was made); desc.cfg.lanes has what
+        runs.  list_batch (2 or 4) has no effect: the force pass loads two
+        list entries ahead, which measured faster than four on every
+        workload."""
         if lanes not in (1, 2, 4, 8) or pair_block % 32 or not 32 <= pair_block <= 256:
             raise ValueError("bad pair-kernel launch shape")
         if self.pairs == "tiled" and lanes != 1:
@@ -494,10 +502,12 @@ class Engine:
             if list_batch not in (2, 4):
                 raise ValueError("list_batch must be 2 or 4")
             self.list_batch = list_batch
+        if exact is not None:
+            self.exact_lanes = bool(exact)
         self.lanes, self.pair_block = lanes, pair_block
         self.pair_tiles = self._make_tiles(pair_block // self._launch_lanes(lanes))
         self._build_desc()
-        # the lists are laid out per lane: record them again
+        # a list's pads depend on the lanes that read it: record them again
         self.invalidate_lists()
 
     def _build_desc(self):

@@ -240,6 +240,8 @@ def test_adjoint_lanes_agree(lanes, block):
     for L, B in ((1, 128), (lanes, block)):
         r = Rollout(arrays, params, fluid_scheme(1), dim=2, dt=1e-5, steps=10,
                     checkpoint_every=5, precision="fp64", adj_lanes=L, adj_pair_block=B)
+        r.adj.set_launch(L, B, exact=True)
+        assert r.adj.desc.cfg.lanes == L
         x = r.forward({0: v0})[0][0]
         g = r.backward({0: (2.0 * x / n, torch.zeros_like(x))})
         grads.append(torch.cat([g[0][0].flatten(), g[0][1].flatten()]))

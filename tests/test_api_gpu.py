@@ -22,7 +22,7 @@ from pysph_b200 import workloads as W
 from helpers import oracle_from
 from pysph_b200.engine import fluid_scheme
 
-pytestmark = pytest.mark.gpu
+pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("thread_rule")]
 Fluid, Solid = base.Fluid, base.Solid
 
 

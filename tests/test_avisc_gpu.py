@@ -20,7 +20,7 @@ import pysph_b200.base.api as base
 import pysph_b200.sph.api as sph
 import pysph_b200.solver.api as solver
 
-pytestmark = pytest.mark.gpu
+pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("thread_rule")]
 Fluid = base.Fluid
 GOLD = os.path.join(os.path.dirname(os.path.abspath(__file__)), "golden", "avisc.npz")
 PROPS = ("x", "y", "z", "u", "v", "w", "m", "h", "rho", "p", "cs")

@@ -11,7 +11,7 @@ from helpers import (oracle_from, oracle_density_eos, oracle_momentum, rel_err,
 from pysph_b200 import workloads as W
 from pysph_b200.engine import Engine, fluid_scheme
 
-pytestmark = pytest.mark.gpu
+pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("thread_rule")]
 
 RHO_TOL = {"fp64": 1e-12, "fp32c": 1e-5}
 ACC_TOL = {"fp64": 1e-10, "fp32c": 1e-4}
@@ -124,7 +124,7 @@ def test_pair_at_support_radius_excluded(precision):
 def test_list_overflow_falls_back_to_the_cell_search(precision, lanes):
     """A 30 x 30 lattice (dx = 0.05, h = 1.3 dx) with a clump of 150 more
     particles within one smoothing length of its centre: their neighbour
-    sets (~180) exceed the list capacity (88 slots, 44 a lane with 2 lanes),
+    sets (~180) exceed the list capacity (96 slots a dest, whatever the lanes),
     so the density pass marks those lists overflowed (count -1) and every
     pass searches their cells instead.  The first evaluation and two
     predictor-corrector steps still match the oracle.  The EOS exponent is
@@ -141,8 +141,10 @@ def test_list_overflow_falls_back_to_the_cell_search(precision, lanes):
     arr = _props(x, y, h=h, m=1000.0 * dx * dx, rho=1000.0)
     params = dict(PARAMS, gamma=1.0)
     scheme = fluid_scheme(1)
-    eng, osys = _check([arr], params, scheme, precision, lanes=lanes, pair_block=128)
-    cnt = eng.fields["nbr_cnt"][:lanes * eng.N].view(lanes, eng.N)
+    eng, osys = _check([arr], params, scheme, precision, lanes=lanes, pair_block=128,
+                       exact_lanes=True)
+    assert eng.desc.cfg.lanes == lanes
+    cnt = eng.fields["nbr_cnt"][:eng.N]
     assert bool((cnt == -1).any()), "no list overflowed"
     for _ in range(2):
         eng.pc_step()

@@ -14,10 +14,10 @@ import torch
 from helpers import (oracle_from, oracle_density_eos, oracle_momentum, rel_err,
                      pairs_from_oracle)
 from pysph_b200 import workloads as W
-from pysph_b200.engine import Engine, continuity_scheme, fluid_scheme, SceneParams
+from pysph_b200.engine import Engine, SceneParams, continuity_scheme, fluid_scheme, lanes_for
 from pysph_b200 import _native as nat
 
-pytestmark = pytest.mark.gpu
+pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("thread_rule")]
 
 RHO_TOL = {"fp64": 1e-12, "fp32c": 1e-5}
 ACC_TOL = {"fp64": 1e-10, "fp32c": 1e-4}
@@ -95,7 +95,8 @@ def test_neighbor_sets_bit_exact(case, stencil):
 @pytest.mark.parametrize("precision", ["fp64", "fp32c"])
 @pytest.mark.parametrize("lanes", [1, 4])
 def test_density_eos(case, precision, lanes):
-    eng, arrays, params, scheme, dim = engine_for(case, precision, lanes=lanes)
+    eng, arrays, params, scheme, dim = engine_for(case, precision, lanes=lanes, exact_lanes=True)
+    assert eng.desc.cfg.lanes == lanes
     osys = oracle_from(arrays, params, scheme, dim)
     osys.update()
     oracle_density_eos(osys, scheme)
@@ -122,7 +123,8 @@ def test_density_eos(case, precision, lanes):
 @pytest.mark.parametrize("precision", ["fp64", "fp32c"])
 @pytest.mark.parametrize("lanes", [1, 8])
 def test_momentum(case, precision, lanes):
-    eng, arrays, params, scheme, dim = engine_for(case, precision, lanes=lanes)
+    eng, arrays, params, scheme, dim = engine_for(case, precision, lanes=lanes, exact_lanes=True)
+    assert eng.desc.cfg.lanes == lanes
     osys = oracle_from(arrays, params, scheme, dim)
     osys.update()
     oracle_density_eos(osys, scheme)
@@ -616,6 +618,7 @@ def test_common_case_loops_match_the_general_loops(case, lists):
     searched every stage) must agree bit for bit."""
     a, arrays, params, scheme, dim = engine_for(case, "fp32c", step_lists=lists)
     b, _, _, _, _ = engine_for(case, "fp32c", step_lists=lists)
+    assert a.desc.cfg.lanes == b.desc.cfg.lanes == lanes_for(a.N, 1)
     for arr in range(b.A):
         b.exchange_in(arr, "h", torch.as_tensor(arrays[arr]["h"], dtype=torch.float64))
     assert not any(t.uniform_h for t in b._scene_host)

@@ -9,7 +9,7 @@ import torch
 from pysph_b200 import workloads as W
 from pysph_b200.engine import Engine, continuity_scheme, fluid_scheme
 
-pytestmark = pytest.mark.gpu
+pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("thread_rule")]
 
 
 def _case(name):

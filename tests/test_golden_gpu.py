@@ -13,7 +13,7 @@ import pytest
 
 from pysph_b200.engine import Engine, fluid_scheme
 
-pytestmark = pytest.mark.gpu
+pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("thread_rule")]
 
 GOLD = os.path.join(os.path.dirname(os.path.abspath(__file__)), "golden")
 PROPS = ("x", "y", "z", "u", "v", "w", "m", "h", "rho", "p", "cs")

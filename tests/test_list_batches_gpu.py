@@ -7,9 +7,10 @@ import pytest
 
 from helpers import oracle_density_eos, oracle_from, oracle_momentum, rel_err
 from pysph_b200 import _native as nat
+from pysph_b200 import engine
 from pysph_b200.engine import Engine, fluid_scheme
 
-pytestmark = pytest.mark.gpu
+pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("thread_rule")]
 
 USE_LIST = 16
 # sums of at most 33 terms: FP64 a few ulp of the largest term, times the
@@ -39,7 +40,9 @@ def test_lists_of_every_length(n, lanes, precision):
                       gravity=(0.0, -9.81, 0.0), dt=1e-5)
         arr = _cluster(n, dim, varying)
         scheme = fluid_scheme(1)
-        eng = Engine([([arr], params)], scheme, dim=dim, precision=precision, lanes=lanes)
+        eng = Engine([([arr], params)], scheme, dim=dim, precision=precision, lanes=lanes,
+                     exact_lanes=True)
+        assert eng.desc.cfg.lanes == lanes
         osys = oracle_from([arr], params, scheme, dim)
         osys.update()
         oracle_density_eos(osys, scheme)
@@ -71,7 +74,8 @@ def test_lists_of_every_length(n, lanes, precision):
 
 @pytest.mark.parametrize("precision", ["fp64", "fp32c"])
 @pytest.mark.parametrize("dim", [2, 3])
-def test_lists_as_long_as_the_capacity(dim, precision):
+@pytest.mark.parametrize("lanes", [1, 2, 4, 8])
+def test_lists_as_long_as_the_capacity(lanes, dim, precision):
     """Every slot of a list can hold an entry: a clump with as many particles
     as there are slots keeps its lists, one more overflows them all (and the
     passes search the cells).  The capacity covers h = 2 dx (66 entries in
@@ -83,7 +87,8 @@ def test_lists_as_long_as_the_capacity(dim, precision):
     for n in (cap, cap + 1):
         arr = _cluster(n, dim, False)
         scheme = fluid_scheme(1)
-        eng = Engine([([arr], params)], scheme, dim=dim, precision=precision)
+        eng = Engine([([arr], params)], scheme, dim=dim, precision=precision, lanes=lanes,
+                     exact_lanes=True)
         osys = oracle_from([arr], params, scheme, dim)
         osys.update()
         oracle_density_eos(osys, scheme)
@@ -100,3 +105,28 @@ def test_lists_as_long_as_the_capacity(dim, precision):
         for a, b in zip(listed[USE_LIST], listed[0]):
             assert rel_err(a, b, scale) <= TOL[precision][1]
         eng.check_status()
+
+
+def test_threads_per_dest():
+    """At least the lanes asked for, more for small engines; exactly as many
+    where the caller says so, for the engine or for one launch shape."""
+    params = dict(dt=1e-5)
+    scenes = [([_cluster(33, 2, False)], params)]
+    kw = dict(dim=2, precision="fp64")
+    for lanes in (1, 2, 4, 8):
+        eng = Engine(scenes, fluid_scheme(1), lanes=lanes, **kw)
+        assert eng.desc.cfg.lanes == engine.lanes_for(33, lanes)
+        eng.set_launch(lanes, 64, exact=True)
+        assert eng.desc.cfg.lanes == eng.lanes == lanes
+        eng.set_launch(lanes, 128)         # as the last call said
+        assert eng.desc.cfg.lanes == lanes
+        eng = Engine(scenes, fluid_scheme(1), lanes=lanes, exact_lanes=True, **kw)
+        assert eng.desc.cfg.lanes == lanes
+        eng.set_launch(lanes, 128, exact=False)
+        assert eng.desc.cfg.lanes == engine.lanes_for(33, lanes)
+    for n, want in ((1, 8), (12500, 8), (12501, 4), (25000, 4), (25001, 2), (50000, 2),
+                    (50001, 1)):
+        if engine.FILL_THREADS:
+            assert engine.lanes_for(n, 1) == want
+        else:
+            assert engine.lanes_for(n, 1) == 1

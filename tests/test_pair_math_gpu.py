@@ -10,7 +10,7 @@ import pytest
 from pysph_b200 import _native as nat
 from pysph_b200.engine import Engine, fluid_scheme
 
-pytestmark = pytest.mark.gpu
+pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("thread_rule")]
 
 
 @pytest.mark.parametrize("lists", [True, False])
