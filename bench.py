@@ -63,7 +63,7 @@ def parse():
     ap.add_argument("--pairs", default="auto", choices=["auto", "lists", "tiled"],
                     help="neighbour lists or shared-memory tiles; default: autotuned")
     ap.add_argument("--list-batch", type=int, default=0,
-                    help="list entries the force pass loads ahead (2 or 4); default: autotuned")
+                    help="no effect (the force pass loads two list entries ahead)")
     return ap.parse_args()
 
 
@@ -323,18 +323,17 @@ def algorithmic_bytes(dim, f32):
 def launch_shape(wl, precision, args, dev, force_tune=False):
     """The engine's launch shape: fixed from the command line, else the
     autotuner's (both pair modes, every cell size / lanes / block / skin)."""
-    if not force_tune and (args.lanes or args.pair_block or args.stencil or args.list_batch
+    if not force_tune and (args.lanes or args.pair_block or args.stencil
                            or args.pairs != "auto"):
         pairs = "lists" if args.pairs == "auto" else args.pairs
         return dict(pairs=pairs, lanes=args.lanes or (4 if wl["dim"] == 3 else 1),
                     pair_block=args.pair_block or 128, stencil=args.stencil or 1,
-                    list_batch=args.list_batch or 4, skin_margin=None), None
+                    skin_margin=None, exact_lanes=True), None
     from pysph_b200.autotune import autotune
     tune = autotune(wl["scenes"], wl["scheme"], wl["dim"], precision, device=dev)
-    shape = {k: tune.get(k) for k in ("pairs", "lanes", "pair_block", "stencil", "list_batch",
-                                      "skin_margin")}
+    shape = {k: tune.get(k) for k in ("pairs", "lanes", "pair_block", "stencil", "skin_margin",
+                                      "exact_lanes")}
     shape["pairs"] = shape["pairs"] or "lists"
-    shape["list_batch"] = shape["list_batch"] or 4
     return shape, tune
 
 
@@ -343,8 +342,8 @@ def make_engine(wl, precision, shape, dev):
     return Engine(wl["scenes"], wl["scheme"], dim=wl["dim"], precision=precision,
                   stencil=shape["stencil"], lanes=shape["lanes"],
                   pair_block=shape["pair_block"], device=dev,
-                  list_batch=shape["list_batch"], skin_margin=shape["skin_margin"],
-                  pairs=shape["pairs"])
+                  skin_margin=shape["skin_margin"], pairs=shape["pairs"],
+                  exact_lanes=bool(shape["exact_lanes"]))
 
 
 def capture_step(eng, stream):
@@ -442,8 +441,8 @@ def run_ours(args, rank, world, local):
            "config": {"workload": args.workload, "description": wl["desc"],
                       "particles": N, "precision": args.precision,
                       "pairs": shape["pairs"], "stencil": shape["stencil"],
-                      "lanes": shape["lanes"], "pair_block": shape["pair_block"],
-                      "list_batch": shape["list_batch"], "skin_margin": eng.skin_margin,
+                      "lanes": eng.desc.cfg.lanes, "pair_block": shape["pair_block"],
+                      "skin_margin": eng.skin_margin,
                       "cuda_graph": graph is not None,
                       "timed_steps": f"steps {start_step + 1}..{start_step + args.steps} of "
                                      "the run from the initial state",
@@ -452,8 +451,7 @@ def run_ours(args, rank, world, local):
            "steps_per_s": steps_per_s,
            "rebins_per_stage": rebins / (2.0 * args.steps),
            "autotune": ({"chosen": {k: tune.get(k) for k in ("pairs", "stencil", "lanes",
-                                                              "pair_block", "list_batch",
-                                                              "skin_margin")},
+                                                              "pair_block", "skin_margin")},
                          "table": tune["table"]} if tune else None),
            "pairs_per_step": pairs / args.steps,
            "gpu_launches": launches_per_step(eng) * args.steps,
@@ -579,7 +577,7 @@ def batched_config(dev, flush, stream, steps=500):
     class A:
         pass
     args = A()
-    args.lanes = args.pair_block = args.stencil = args.list_batch = 0
+    args.lanes = args.pair_block = args.stencil = 0
     args.pairs = "auto"
     wl = workload("batched")
     out = {"workload": wl["desc"]}

@@ -3,11 +3,12 @@
 For a workload it times whole predictor-corrector steps for every candidate
 of cell size (stencil R: cell = support / R), lanes per dest particle and
 threads per block, with the neighbour lists and (2D FP32C summation
-density) with the shared-memory tiles, and returns the fastest.  On that shape it then tries
-the force pass's load-ahead depth (FP32C) and the skin of the kept
-neighbour lists: a wider skin means longer lists but fewer rebins, which
-pays where particles move fast.  Results are cached per (dim, precision,
-particle-count bucket, scene-count bucket), in memory and, when
+density) with the shared-memory tiles, and returns the fastest.  The lanes
+are exact: every candidate runs as many threads per dest as it says, and the
+result asks for them with exact_lanes.  On that shape it then tries the skin
+of the kept neighbour lists: a wider skin means longer lists but fewer
+rebins, which pays where particles move fast.  Results are cached per (dim,
+precision, particle-count bucket, scene-count bucket), in memory and, when
 PYSPH_B200_TUNE_CACHE names a file, in that JSON file.
 """
 from __future__ import annotations
@@ -75,8 +76,8 @@ def tiled_ok(scheme, dim, precision, variable_h=False) -> bool:
 
 def autotune(scenes, scheme, dim, precision="fp32c", device=None, stencils=STENCILS,
              lanes=LANES, blocks=BLOCKS, steps=4, force=False, tiled=True):
-    """Best {"pairs", "stencil", "lanes", "pair_block", "ms_per_step"} plus the
-    table of every candidate timed."""
+    """Best {"pairs", "stencil", "lanes", "exact_lanes", "pair_block",
+    "skin_margin", "ms_per_step"} plus the table of every candidate timed."""
     _load()
     n = sum(len(a["x"]) for arrays, _ in scenes for a in arrays)
     key = _key(dim, precision, n, len(scenes))
@@ -90,11 +91,11 @@ def autotune(scenes, scheme, dim, precision="fp32c", device=None, stencils=STENC
             for B in blocks:
                 if B % L or B // L < 8:
                     continue
-                eng.set_launch(L, B)
+                eng.set_launch(L, B, exact=True)
                 ms = time_steps(eng, steps)
                 eng.check_status()
-                table.append({"pairs": "lists", "stencil": R, "lanes": L, "pair_block": B,
-                              "ms_per_step": ms})
+                table.append({"pairs": "lists", "stencil": R, "lanes": L,
+                              "exact_lanes": True, "pair_block": B, "ms_per_step": ms})
         del eng
         if tiled and tiled_ok(scheme, dim, precision):
             eng = Engine(scenes, scheme, dim=dim, precision=precision, stencil=R,
@@ -105,37 +106,29 @@ def autotune(scenes, scheme, dim, precision="fp32c", device=None, stencils=STENC
                 eng.set_launch(1, B)
                 ms = time_steps(eng, steps)
                 eng.check_status()
-                table.append({"pairs": "tiled", "stencil": R, "lanes": 1, "pair_block": B,
-                              "ms_per_step": ms})
+                table.append({"pairs": "tiled", "stencil": R, "lanes": 1,
+                              "exact_lanes": True, "pair_block": B, "ms_per_step": ms})
             del eng
     best = min(table, key=lambda r: r["ms_per_step"])
-    best = dict(best, list_batch=4)
+    shape = {k: best[k] for k in ("pairs", "stencil", "lanes", "exact_lanes", "pair_block")}
     if precision == "fp32c" and best["pairs"] == "lists":
-        # load-ahead depth of the force pass's list loop, on the best shape
-        eng = Engine(scenes, scheme, dim=dim, precision=precision, stencil=best["stencil"],
-                     lanes=best["lanes"], pair_block=best["pair_block"], device=device,
-                     list_batch=2)
+        # the best shape once more, on an engine of its own: beside its first
+        # time it shows how far the table's times scatter
+        eng = Engine(scenes, scheme, dim=dim, precision=precision, device=device, **shape)
         ms = time_steps(eng, steps)
         eng.check_status()
-        table.append({"pairs": "lists", "stencil": best["stencil"], "lanes": best["lanes"],
-                      "pair_block": best["pair_block"], "list_batch": 2, "ms_per_step": ms})
-        if ms < best["ms_per_step"]:
-            best = dict(table[-1])
+        table.append(dict(shape, ms_per_step=ms))
         del eng
     # the skin, on enough steps for the rebins to show (fresh engines, so
     # every candidate starts from the same state)
     skin_table = []
     for skin in SKINS:
-        eng = Engine(scenes, scheme, dim=dim, precision=precision, stencil=best["stencil"],
-                     lanes=best["lanes"], pair_block=best["pair_block"], device=device,
-                     list_batch=best.get("list_batch", 4), skin_margin=skin,
-                     pairs=best["pairs"])
+        eng = Engine(scenes, scheme, dim=dim, precision=precision, device=device,
+                     skin_margin=skin, **shape)
         ms = time_steps(eng, 4 * steps, warm=steps)
         eng.check_status()
-        skin_table.append(dict(pairs=best["pairs"], stencil=best["stencil"], lanes=best["lanes"],
-                               pair_block=best["pair_block"],
-                               list_batch=best.get("list_batch", 4), skin_margin=skin,
-                               ms_per_step=ms))
+        # (list_batch has no effect; results keep the key)
+        skin_table.append(dict(shape, list_batch=4, skin_margin=skin, ms_per_step=ms))
         del eng
     table.extend(skin_table)
     best = dict(min(skin_table, key=lambda r: r["ms_per_step"]))

@@ -492,6 +492,31 @@ def test_autotune_returns_a_timed_shape(tmp_path, monkeypatch):
     T._cache.clear()
 
 
+def test_autotune_times_the_shapes_that_it_reports(monkeypatch):
+    """Every candidate runs as many threads per dest as its row says, and no
+    two candidates but the repeated winner are the same program."""
+    from pysph_b200 import autotune as T
+    monkeypatch.delenv("PYSPH_B200_TUNE_CACHE", raising=False)
+    T._cache.clear()
+    ran = []
+    time_steps = T.time_steps
+
+    def spy(eng, *a, **k):
+        ran.append((eng.pairs, eng._stencil, eng.desc.cfg.lanes, eng.pair_block, eng.skin_margin))
+        return time_steps(eng, *a, **k)
+    monkeypatch.setattr(T, "time_steps", spy)
+    arrays, params, scheme, dim = drop(dx=0.05)
+    res = T.autotune([(arrays, dict(params, dt=1e-5))], scheme, dim, "fp32c", blocks=(64, 128),
+                     stencils=(1,), steps=2)
+    T._cache.clear()
+    rows = [(r["pairs"], r["stencil"], r["lanes"], r["pair_block"],
+             r.get("skin_margin", 0.15)) for r in res["table"]]
+    assert ran == rows and all(r["exact_lanes"] for r in res["table"])
+    shapes = [r for r in rows[:-len(T.SKINS)]]
+    assert len(shapes) - len(set(shapes)) <= 1
+    assert {r[2] for r in shapes if r[0] == "lists"} == set(T.LANES)
+
+
 def test_euler_step_graph_replays_like_eager_steps():
     """A captured Euler step (one stage) keeps the record copies in place, so
     its replays match eager steps."""
