@@ -424,6 +424,8 @@ class Engine:
             self.list_cap += -self.list_cap % 32
         if self.list_cap:
             f["nbr"] = torch.zeros(self.list_cap * N, **i32)
+            # one count per dest, in the first N words (the rest only keeps the
+            # size that readers of per-thread counts expect)
             f["nbr_cnt"] = torch.zeros(8 * N, **i32)
         else:
             f["nbr"] = f["nbr_cnt"] = None
