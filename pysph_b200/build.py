@@ -5,8 +5,8 @@
 Every .cu under csrc/ is compiled by nvcc for sm_100a only, in parallel, and
 linked into pysph_b200/_lib/libsphb.so with the CUDA runtime linked
 statically, so the library carries no dependency beyond the driver.  The
-benchmark's FMA-rate probe (probe/) is built into its own
-_lib/libsphb_probe.so.
+probes (probe/: the benchmark's FMA rates, the pair arithmetic on arrays for
+its test) are built into their own _lib/libsphb_probe.so.
 """
 from __future__ import annotations
 
@@ -66,17 +66,16 @@ def _compile(src, extra):
     return obj, ""
 
 
-PROBE_SRC = os.path.join(HERE, "probe", "sphb_fma_probe.cu")
+PROBE_SRC = [os.path.join(HERE, "probe", f)
+             for f in ("sphb_fma_probe.cu", "sphb_math_probe.cu")]
 PROBE_LIB = os.path.join(LIBDIR, "libsphb_probe.so")
 
 
 def build_probe(force: bool = False) -> str:
-    """The benchmark's FMA-rate probe, a library of its own (not part of
-    libsphb.so)."""
+    """The probes, a library of their own (not part of libsphb.so)."""
     os.makedirs(LIBDIR, exist_ok=True)
-    if force or _stale(PROBE_LIB, [PROBE_SRC, __file__]):
-        cmd = [nvcc(), "-shared", PROBE_SRC, "-o", PROBE_LIB + ".tmp"] + ARCH + [
-            "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",
+    if force or _stale(PROBE_LIB, PROBE_SRC + _headers() + [__file__]):
+        cmd = [nvcc(), "-shared"] + PROBE_SRC + ["-o", PROBE_LIB + ".tmp"] + NVCC_FLAGS + [
             "-cudart", "static"]
         subprocess.check_call(cmd)
         os.replace(PROBE_LIB + ".tmp", PROBE_LIB)

@@ -463,7 +463,8 @@ k_force(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask,
             const double kf = Kern<KT>::template norm<DIM>();
             const double alp_k = alpha * hk, bet2_k = 2.0 * beta * hk * hk;
             const double ihk = 1.0 / hk;
-            const double fihk = DIM == 2 ? kf * ihk * ihk * ihk : kf * ihk * ihk * ihk * ihk;
+            const double fack = (DIM == 2 ? 1.0 / (hk * hk) : 1.0 / (hk * hk * hk)) * kf;
+            const double fihk = fack / hk;
             // with one h in the scene the symmetric set and the averaged
             // kernels are the plain ones
             const bool vh = sc.variable_h != 0, hks = sc.hks != 0;
@@ -521,28 +522,32 @@ k_force(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask,
                         const bool rate_on = in && CONT && (rm & r.bit);
                         const bool xs_on = in && CONT && (xm & r.bit);
                         const double hab = UH ? hk : 0.5 * (hk + r.h);
-                        const double ir = inv_dist(r2);
+                        double ir;
+                        const double rr = dist_pair(r2, ir);
                         // grad W / r (and W for XSPH) at h_ab, or with hks the
                         // means of the values at h_a and h_b (pressure_funcs.pyx:
                         // 371-381)
                         double gw, w = 0.0;
                         if (UH) {
-                            const double q = mul_pair(r2 * ir, ihk);
+                            const double q = over_h(rr, hk, ihk);
                             gw = Kern<KT>::template gw_in<false>(q, ir, ihk, fihk);
-                            if (CONT) w = Kern<KT>::template w_in<false>(q, fihk * hk);
+                            if (CONT) w = Kern<KT>::template w_in<false>(q, fack);
                         } else {
-                            const double rr = r2 * ir;
+                            auto eval = [&](double hs, double ih, double fac, double fih,
+                                            double &wh) {
+                                const double q = over_h(rr, hs, ih);
+                                if (CONT) wh = Kern<KT>::template w_in<true>(q, fac);
+                                return Kern<KT>::template gw_in<true>(q, ir, ih, fih);
+                            };
                             auto at = [&](double hs, double &wh) {
                                 const double ih = rcp_pair(hs);
-                                const double fih = DIM == 2 ? kf * ih * ih * ih
-                                                            : kf * ih * ih * ih * ih;
-                                const auto q = mul_pair(rr, ih);
-                                if (CONT) wh = Kern<KT>::template w_in<true>(q, fih * hs);
-                                return Kern<KT>::template gw_in<true>(q, ir, ih, fih);
+                                const double fac =
+                                    (DIM == 2 ? rcp_pair(hs * hs) : rcp_pair(hs * hs * hs)) * kf;
+                                return eval(hs, ih, fac, fac * ih, wh);
                             };
                             double wa = 0.0, wb = 0.0;
                             if (hks) {
-                                gw = 0.5 * (at(hk, wa) + at(r.h, wb));
+                                gw = 0.5 * (eval(hk, ihk, fack, fihk, wa) + at(r.h, wb));
                                 w = 0.5 * (wa + wb);
                             } else {
                                 gw = at(hab, w);

@@ -28,8 +28,9 @@ namespace sphb {
 // straight run of instructions, which the compiler interleaves.  FP32: the
 // hardware approximation.  FP64: the hardware's seed (relative error below
 // 2^-19), then one third-order step from the binomial series of 1 / (1 - e)
-// and 1 / sqrt(1 - e) in the seed's residual e; the results are within 2
-// units in the last place (tests/test_pair_math_gpu.py).
+// and 1 / sqrt(1 - e) in the seed's residual e.  Largest errors over 4 million
+// mantissas, in units of the last place: 1 / x 0.51, r 0.75, 1 / r 0.99, r / h
+// 0.50 (tests/test_pair_math_gpu.py has the bounds).
 __device__ __forceinline__ float rcp_pair(float x)
 {
     float y;
@@ -52,13 +53,19 @@ __device__ __forceinline__ float rsqrt_pair(float x)
     return y;
 }
 
-__device__ __forceinline__ double rsqrt_pair(double x)
+// r and 1 / r from r^2, both from the one series: y (1 + p) and r^2 y (1 + p)
+// with y the seed.  The rounding d of t = r^2 y enters each as d / 2, beside
+// the last rounding.  Finite at r = 0, where r is 1e-100.
+__device__ __forceinline__ double dist_pair(double r2, double &ir)
 {
+    const double x = fmax(r2, 1e-200);
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double t = x * y, tl = fma(x, y, -t);   // x y exactly
-    const double e = fma(-tl, y, fma(-t, y, 1.0));
-    return fma(y, e * fma(0.375, e, 0.5), y);
+    const double t = x * y;
+    const double e = fma(-t, y, 1.0);
+    const double p = e * fma(0.375, e, 0.5);
+    ir = fma(y, p, y);
+    return fma(t, p, t);
 }
 
 // A product that no later sum contracts into an FMA.  The FP32C pair loops
@@ -68,9 +75,16 @@ __device__ __forceinline__ double rsqrt_pair(double x)
 __device__ __forceinline__ float mul_pair(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double mul_pair(double a, double b) { return __dmul_rn(a, b); }
 
-// 1 / r from r^2; finite at r = 0, where r^2 times it is 0.
+// FP32: 1 / r from r^2; finite at r = 0, where r^2 times it is 0.
 __device__ __forceinline__ float inv_dist(float r2) { return rsqrt_pair(fmaxf(r2, 1e-30f)); }
-__device__ __forceinline__ double inv_dist(double r2) { return rsqrt_pair(fmax(r2, 1e-200)); }
+
+// q = r / h from r, h and 1 / h.  FP64: with the product's residual added back,
+// so that q is rounded as a division rounds it.
+__device__ __forceinline__ double over_h(double r, double h, double ih)
+{
+    const double q = r * ih;
+    return fma(fma(-h, q, r), ih, q);
+}
 
 template <int KT>
 struct Kern;

@@ -1,13 +1,17 @@
 """The FP64 pair arithmetic (seeded reciprocals and reciprocal square roots
-in place of divisions) to a few units in the last place: scenes of one pair
-each, over six orders of magnitude of h and every distance within the
-support, densities and accelerations against numpy."""
+in place of divisions): the functions themselves against 80-bit arithmetic, to
+units in the last place; and scenes of one pair each, over six orders of
+magnitude of h and every distance within the support, densities and
+accelerations against numpy."""
+import ctypes
 import math
 
 import numpy as np
 import pytest
+import torch
 
 from pysph_b200 import _native as nat
+from pysph_b200 import build
 from pysph_b200.engine import Engine, fluid_scheme
 
 pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("thread_rule")]
@@ -61,3 +65,56 @@ def test_one_pair_per_scene(lists):
         cond = np.where(dot < 0, np.minimum(cond, 1e3), 1)[:, None]
         assert np.max(np.abs(acc[:, a] - want) / (scale * cond)) < 2e-14
     eng.check_status()
+
+
+def _probe(which, a, b=None):
+    fn = ctypes.CDLL(build.PROBE_LIB).sphb_math_probe
+    p = ctypes.c_void_p
+    fn.argtypes = [ctypes.c_int, ctypes.c_int, p, p, p, p, p]
+    dev = torch.device("cuda", torch.cuda.current_device())
+    a = torch.as_tensor(a, device=dev)
+    b = None if b is None else torch.as_tensor(b, device=dev)
+    out, out2 = torch.empty_like(a), torch.empty_like(a)
+    assert fn(which, a.numel(), a.data_ptr(), None if b is None else b.data_ptr(),
+              out.data_ptr(), out2.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    return out.cpu().numpy(), out2.cpu().numpy()
+
+
+def _ulps(got, want):
+    """Largest error in units in the last place (want: 80 bits, 11 more than
+    the unit; its own rounding is 2^-12 of one)."""
+    return float(np.max(np.abs(got.astype(np.longdouble) - want)
+                        / np.spacing(np.abs(want.astype(np.float64)))))
+
+
+def _numbers(rng, n, lo, hi):
+    """Random mantissas and the ends of the mantissa's range, exponents of
+    lo .. hi."""
+    m = np.concatenate([rng.uniform(1, 2, n - 64), 1 + np.spacing(1.0) * np.arange(32),
+                        2 - np.spacing(1.0) * np.arange(1, 33)])
+    return np.ldexp(m, rng.integers(lo, hi, n))
+
+
+def test_reciprocals_distances_and_quotients():
+    """The seeds are within 2^-19 of the result (e below 2^-19, 2^-18 for the
+    square root).  Reciprocal: half a unit of the last FMA and e^3 < 2^-57.
+    Distance and its reciprocal: half a unit, half the rounding of t (at most
+    half a unit more) and 5/16 e^3 < 2^-55.  Quotient: half a unit, the residual
+    being exact and its own factor off by 2^-52 of it."""
+    L = np.longdouble
+    rng = np.random.default_rng(5)
+    n = 1 << 20
+    a = _numbers(rng, n, -300, 300)
+    assert _ulps(_probe(0, a)[0], 1 / a.astype(L)) <= 0.5 + 2.0 ** -4 + 2.0 ** -10
+    assert _ulps(_probe(0, -a)[0], -1 / a.astype(L)) <= 0.5 + 2.0 ** -4 + 2.0 ** -10
+    r2 = _numbers(rng, n, -600, 600)
+    r, ir = _probe(1, r2)
+    s = np.sqrt(r2.astype(L))
+    assert _ulps(r, s) <= 1.0 + 2.0 ** -2 + 2.0 ** -10
+    assert _ulps(ir, 1 / s) <= 1.0 + 2.0 ** -2 + 2.0 ** -10
+    h = _numbers(rng, n, -40, 40)
+    x = h * rng.uniform(0.0, 3.0, n)
+    assert _ulps(_probe(2, x, h)[0], x.astype(L) / h) <= 0.5 + 2.0 ** -10
+    # a particle with itself: a finite reciprocal, a distance far below any h
+    r, ir = _probe(1, np.zeros(1))
+    assert 0 <= r[0] <= 1e-99 and np.isfinite(ir[0])
