@@ -320,7 +320,12 @@ constexpr int record_smem(int threads)
 // dests' runs and the accepted ones are numbered with one warp-wide ballot.
 // (A ballot over each dest's threads alone splits the warp: 45 -> 91 us, the
 // recording pass of an 86k-particle FP64 dam break with 2 threads a dest,
-// against 49 us this way.)
+// against 49 us this way.)  Taken one at a time, a candidate's loads wait for
+// the test of the last one.  Recording passes with 1 / 2 / 4 candidates a
+// turn: 2 threads, 100k FP64 drop 39.6 / 36.4 / 34.1 us, 300k 3D lattice 342 /
+// 325 / 322; 4 threads, 20k FP64 drop 14.4 / 13.7 / 13.4, 125k FP64 lattice
+// 253 / 219 / 219; 8 threads, 125k FP32C lattice 206 / 198 / 201, 300k FP64
+// 443 / 430 / 451.
 template <int DIM, int R, int LANES, typename Accept>
 __device__ __forceinline__ int record_list(const sphb_engine &e, uint32_t *nbr, int2 *rows, int k,
                                            bool active, uint32_t src_mask, int cell_base,
@@ -329,6 +334,7 @@ __device__ __forceinline__ int record_list(const sphb_engine &e, uint32_t *nbr, 
 {
     constexpr int NR = 2 * R + 1;
     constexpr float RC2 = (R + 1e-3f) * (R + 1e-3f);
+    constexpr int K = LANES == 2 ? 4 : 2;
     const int lane = threadIdx.x & (LANES - 1);
     const int nd = blockDim.x / LANES;           // dests of the block
     rows += threadIdx.x / LANES;
@@ -384,16 +390,24 @@ __device__ __forceinline__ int record_list(const sphb_engine &e, uint32_t *nbr, 
             };
             advance(lane);
             while (__any_sync(0xffffffffu, i < NR)) {
-                bool take = false;
-                const int jc = j, dy = i - R;
-                int o = 0;
-                if (i < NR) {
-                    // the x offset from the candidate's own cell
-                    o = __ldg(cell + j) - (local + (dz * n[1] + dy) * n[0]);
-                    take = accept(j, o, dy, dz);
-                    advance(LANES);
+                // K candidates a turn, their loads in flight together (past
+                // the end: particle 0, not taken)
+                int jc[K], dy[K], o[K];
+                bool take[K];
+#pragma unroll
+                for (int c = 0; c < K; ++c) {
+                    take[c] = i < NR;
+                    jc[c] = take[c] ? j : 0;
+                    dy[c] = i - R;
+                    if (i < NR) advance(LANES);
                 }
-                list.put(take, jc, o, dy, dz);
+#pragma unroll
+                for (int c = 0; c < K; ++c)   // the x offset from its own cell
+                    o[c] = __ldg(cell + jc[c]) - (local + (dz * n[1] + dy[c]) * n[0]);
+#pragma unroll
+                for (int c = 0; c < K; ++c) take[c] = accept(jc[c], o[c], dy[c], dz) && take[c];
+#pragma unroll
+                for (int c = 0; c < K; ++c) list.put(take[c], jc[c], o[c], dy[c], dz);
             }
         }
     }
