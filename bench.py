@@ -223,30 +223,29 @@ def replica_result(ms_per_rank, pairs_per_rank, steps, world, device="cuda"):
 
 # DRAM bytes (read + write) per launch from `ncu --set full` on the bench's
 # own workload (the dam break, FP32C, lists, 1 lane, 256-thread blocks,
-# cells of half the reach, force list batches of 2; the force pass with the
-# integrator stage fused into it): the mean of the two captured launches of
-# each kernel (profiles/k_force_dam_break_fp32c.md,
-# profiles/k_density_dam_break_fp32c.md)
-NCU_TRAFFIC = {("dam_break", "fp32c", "lists", "force"): 0.5 * ((73.27e6 + 3.05e6) +
-                                                                (63.03e6 + 4.72e6)),
+# cells of half the reach; the force pass with the integrator stage fused
+# into it): the mean of the two captured launches of each kernel
+# (profiles/k_force_dam_break_fp32c.md, profiles/k_density_dam_break_fp32c.md)
+NCU_TRAFFIC = {("dam_break", "fp32c", "lists", "force"): 0.5 * ((73.26e6 + 3.58e6) +
+                                                                (63.03e6 + 4.06e6)),
                ("dam_break", "fp32c", "lists", "density"): 44.90e6 + 0.03e6,
                ("dam_break", "fp32c", "lists", "pc_stage"): 17.951e6 + 0.000256e6,
                # the 256 drops (block 128, the rest as above;
                # profiles/k_pairs_batched_fp32c.md)
-               ("batched", "fp32c", "lists", "force"): 583.87e6 + 257.02e6,
-               ("batched", "fp32c", "lists", "density"): 389.22e6 + 43.41e6}
+               ("batched", "fp32c", "lists", "force"): 561.09e6 + 253.24e6,
+               ("batched", "fp32c", "lists", "density"): 389.36e6 + 39.82e6}
 
 
 # FP32 work of one launch from the same capture: flops = 2 FFMA + FADD +
 # FMUL + 4 FFMA2 + 2 FADD2 + 2 FMUL2 (sm__sass_thread_inst_executed_op_*;
 # no paired instructions were issued), and the fraction of cycles the
 # schedulers issued (smsp__issue_active.avg.pct_of_peak_sustained_active)
-NCU_FP32 = {("dam_break", "fp32c", "lists", "force"): {"flops": 396.3e6, "issue_active": 0.587},
-            ("dam_break", "fp32c", "lists", "density"): {"flops": 225.6e6,
-                                                         "issue_active": 0.663},
-            ("batched", "fp32c", "lists", "force"): {"flops": 3507.2e6, "issue_active": 0.585},
-            ("batched", "fp32c", "lists", "density"): {"flops": 1934.9e6,
-                                                       "issue_active": 0.801}}
+NCU_FP32 = {("dam_break", "fp32c", "lists", "force"): {"flops": 410.9e6, "issue_active": 0.503},
+            ("dam_break", "fp32c", "lists", "density"): {"flops": 264.4e6,
+                                                         "issue_active": 0.605},
+            ("batched", "fp32c", "lists", "force"): {"flops": 3610.7e6, "issue_active": 0.590},
+            ("batched", "fp32c", "lists", "density"): {"flops": 2265.3e6,
+                                                       "issue_active": 0.709}}
 
 
 def fma_peaks(dev):
@@ -506,12 +505,14 @@ def roofline(eng, workload_name, precision, flush, stream, rebins_per_stage):
             "peak": hbm, "peak_kind": which, "unit": "GB/s",
             "frac": round(ach / hbm, 4), "traffic": traffic,
             "traffic_note": ("dram__bytes_read.sum + dram__bytes_write.sum per launch, one ncu "
-                             "capture of this workload and launch shape") if traffic else None,
+                             "capture of this workload, on the launch shape that profiles/ "
+                             "names") if traffic else None,
             "per_kernel_ms": {k: round(v, 5) for k, v in kern.items()},
             "per_stage_ms": {k: round(v, 5) for k, v in per_stage.items()},
             "bytes_per_particle": byts}
-    # the pair passes are bound by instruction issue: their FP32 flop rate
-    # against the measured FMA peak, and the issue-active fraction ncu saw
+    # the pair passes are bound by the latency of their gathers and by issue,
+    # not by DRAM: their FP32 flop rate against the measured FMA peak, and the
+    # issue-active fraction ncu saw
     peaks_c = fma_peaks(eng.device)
     fp = NCU_FP32.get((workload_name, precision, eng.pairs, dominant))
     if fp:
