@@ -297,9 +297,10 @@ class NNPSManager:
 class Particles:
     """A collection of particle arrays (S/base/particles.py:35-227).
 
-    precision: 'fp64' (default: the reference's arithmetic) or 'fp32c' (FP32
-    pair sums with Kahan compensation, FP64 state); arrays created with
-    cl_precision='single' select 'fp32c' by default."""
+    precision: 'fp64' (default: float64 throughout, the reference's neighbour
+    predicate operation for operation) or 'fp32c' (FP32 pair sums with Kahan
+    compensation, FP64 state); arrays created with cl_precision='single'
+    select 'fp32c' by default."""
 
     def __init__(self, arrays=(), in_parallel=False, variable_h=False,
                  load_balancing=True, locator_type=SPHNeighborLocator,

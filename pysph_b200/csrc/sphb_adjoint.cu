@@ -120,9 +120,9 @@ k_force_vjp(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask, 
     // array decides the dest-role sources, mom_src of the neighbour's array
     // the source role
     const uint32_t all = (1u << A) - 1u;
-    // the lists of the density pass (recorded one lane per particle) hold
-    // every pair of both roles when h is uniform (the predicate is then
-    // symmetric)
+    // the lists of the density pass (one row per dest, which its threads read
+    // in turn) hold every pair of both roles when h is uniform (the predicate
+    // is then symmetric)
     const bool use_list = sc.uniform_h && e.cfg.rho_src[a] != 0u && e.cfg.lanes == LANES &&
                           e.f.list_cap > 0 && e.f.nbr && e.f.nbr_cnt;
     if (active) traverse<DIM, R, LANES>(
@@ -288,9 +288,9 @@ k_density_vjp(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask
     int cx, cy, cz;
     cell_coords(e.f.cell[k], n, cx, cy, cz);
     const uint32_t all = (1u << A) - 1u;
-    // the lists of the density pass (recorded one lane per particle) hold
-    // every pair of both roles when h is uniform (the predicate is then
-    // symmetric)
+    // the lists of the density pass (one row per dest, which its threads read
+    // in turn) hold every pair of both roles when h is uniform (the predicate
+    // is then symmetric)
     const bool use_list = sc.uniform_h && e.cfg.rho_src[a] != 0u && e.cfg.lanes == LANES &&
                           e.f.list_cap > 0 && e.f.nbr && e.f.nbr_cnt;
     if (active) traverse<DIM, R, LANES>(

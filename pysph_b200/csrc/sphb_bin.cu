@@ -988,14 +988,14 @@ __device__ void copy_back_run(const sphb_engine &e, int cur, int mi, int t0, int
 // when the cells are kept; the gathered state then goes back to buf[cur].
 //
 // A rebin of few particles is a chain of latencies, above all the barriers
-// (~2.5 us each with 296 blocks): resetting the boxes, the decision's
-// commit, the grids and the chunk totals used to be phases of their own (ten
-// barriers).  The accumulators of the box and the totals are now left clear
-// by the rebin before, the commit waits for the first barrier, and every
-// block sets up the grids for itself (more than 256 scenes: block 0 alone,
-// one more barrier): a full
-// rebin 35 -> 27 us at 5k particles, 38 -> 31 us at 60k, 85 -> 81 us at 332k, 296 -> 285 us for
-// 256 drops (2.9M).
+// (~2.5 us each with 296 blocks), so the reset of the boxes, the decision's
+// commit, the grids and the chunk totals are no phases of their own: a rebin
+// leaves the accumulators of the box and the totals clear for the next one,
+// the commit waits for the first barrier, and every block sets up the grids
+// for itself (more than 256 scenes: block 0 alone, one more barrier).  A full
+// rebin with those phases (ten barriers) and without: 35 and 27 us at 5k
+// particles, 38 and 31 us at 60k, 85 and 81 us at 332k, 296 and 285 us for 256
+// drops (2.9M).
 template <int DIM, bool F32>
 __global__ void __launch_bounds__(SPHB_ELEM_TILE)
 k_rebin(const __grid_constant__ sphb_engine e, int cur, int flags)

@@ -30,7 +30,7 @@ namespace sphb {
 
 // Everything after the pair sums of dest k: its outputs (non-LocalReal
 // dests get 0), gravity, dt_fac, the per-scene CFL maxima, the integrator
-// stage fused into the epilogue (FP32C) and the pair count.  Every thread
+// stage fused into the epilogue and the pair count.  Every thread
 // of the block calls it (block reductions inside); acc, dtf, drho and xs
 // are valid in lane 0 of each dest; visc: the pass has a viscous term
 // and writes dt_fac.
@@ -147,10 +147,11 @@ __device__ __forceinline__ void force_finish(const sphb_engine &e, int cur, int 
 // (1,109 us per 10 steps of 146k particles, 80 registers 1,122, 128 1,163).
 // FP64 in 2D 96: 16% of its 128-register time on an 86k-particle dam break
 // was a second wave of blocks (1,304 -> 1,248 us per 10 steps).
-// The FP64 pair was bound by its own latency: one neighbour at a time, four
-// dependent rounds of loads, eight divisions and a square root in branches.
-// With a batch's fields loaded together, P / rho^2 kept per particle, and no
-// division or branch in a pair, the pass goes 134 -> 42 us on that dam break.
+// The FP64 pair is bound by the latency of its gathers and by issue: a batch's
+// fields are loaded together, P / rho^2 is kept per particle, and no division
+// or branch stands in a pair (one neighbour at a time with four dependent
+// rounds of loads, eight divisions and a square root in branches: 134 us on
+// that dam break, against 42).
 template <int DIM, bool F32, bool CONT>
 constexpr int force_regs()
 {
@@ -318,8 +319,7 @@ k_force(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask,
                         // r = 0 (self) gives q = 0 and a finite gradient times r_ab = 0
                         const float ir = inv_dist(r2);
                         // grad W / r (and W for XSPH) at h_ab, or with hks the means
-                        // of the values at h_a and h_b: one evaluation in a loop
-                        // keeps the register count of the uniform-h path
+                        // of the values at h_a and h_b
                         float gw, w = 0.f;
                         if (UH) {
                             const float q = mul_pair(r2 * ir, ihk);

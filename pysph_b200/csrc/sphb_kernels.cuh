@@ -3,18 +3,19 @@
 // Kern<KT> (KT = SPHB_KERNEL_*) gives, for one kernel type:
 //   norm<DIM>()             _fac(1.0), the normalisation at h = 1
 //   w_bf(q, fac)            W = fac val(q), branch-free (every piece
-//                           computed, one selected) for the list loops
+//                           computed, one selected): the tiled passes
 //   gw_bf(q, ir, ih, fac_ih) dW/dr / r in the reference's sign convention,
 //                           so grad_a W = (x_a - x_b) gw
-//   w_in, gw_in<CLAMP>      the same for the pair loops; without CLAMP inside
-//                           the support only.  gw_in keeps every factor of h
-//                           outside the polynomial: with one h in the scene
-//                           they are constants of the loop
+//   w_in, gw_in<CLAMP>      the same for the list passes and their cell
+//                           searches; without CLAMP inside the support only.
+//                           gw_in keeps every factor of h outside the
+//                           polynomial: with one h in the scene they are
+//                           constants of the loop
 // with fac = norm<DIM>() / h^DIM, ih = 1 / h, ir = 1 / r, fac_ih = fac ih,
 // for T = float and double.  No form divides: the pair loops take one
 // reciprocal square root per pair and, with one h in the scene, the dest's
-// 1 / h.  For r = 0 they see a finite ir (inv_dist); every caller multiplies
-// gw by r_ab = 0 there.
+// 1 / h.  For r = 0 they see a finite ir (inv_dist, dist_pair); every caller
+// multiplies gw by r_ab = 0 there.
 
 #pragma once
 

@@ -249,7 +249,8 @@ class Engine:
         # symmetric neighbour sets r < radius_scale max(h_a, h_b)
         # (VarHNbrParticleLocator) instead of r < radius_scale h_a
         self.variable_h = bool(variable_h)
-        # run the integrator stage in the force pass's epilogue (FP32C)
+        # run the integrator stage in the force pass's epilogue (see
+        # fuses_stage)
         self.fuse_stage = bool(fuse_stage)
         self.force_mode = 0       # 0 MomentumEquation, 1 SPHPressureGradient
         self.tait_only_mask = 0    # Tait dests that are not SPHRho dests
