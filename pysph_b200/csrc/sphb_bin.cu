@@ -265,8 +265,14 @@ __device__ __forceinline__ long long scene_grid(const sphb_engine &e, int s, Sce
             g.n[d] = (int)(fhi - flo) + 1 + 2 * R;
         }
     }
-    const long long need = (long long)e.cfg.num_arrays * g.n[0] * g.n[1] * g.n[2];
-    if (bad || need > e.cfg.cell_capacity) bad = true;
+    // axis by axis: particles far apart in 3D (10^8 cells an axis) would
+    // overflow 64 bits, and a product that wrapped below the capacity would
+    // send keys outside the tables
+    long long need = e.cfg.num_arrays;
+    for (int d = 0; d < 3 && !bad; ++d) {
+        need *= g.n[d];
+        bad = need > e.cfg.cell_capacity;
+    }
     return bad ? 0 : need;
 }
 

@@ -1,5 +1,6 @@
-"""The rebin's launch follows its work: particles and cells.  The number of
-blocks is read from a captured graph."""
+"""The rebin's launch follows its work (particles and cells; the number of
+blocks is read from a captured graph), and boxes of any size that do not fit
+the cell table are reported."""
 import numpy as np
 import pytest
 import torch
@@ -53,3 +54,33 @@ def test_small_engines_wait_for_few_blocks(cells):
     eng = _engine(1000, 10.0, 2, cell_capacity=cells)
     assert _rebin_blocks(eng) == [max(4, -(-cells // 4096))]
     eng.check_status()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32c"])
+@pytest.mark.parametrize("cells", [2.1e6, 2.0 ** 21 - 8, 4.0e6, 3.0e7, 9.9e7])
+def test_boxes_whose_cells_overflow_64_bits_are_reported(cells, precision):
+    """cells an axis in 3D: 2.1e6 cubed is past 2^63, so a 64-bit product is
+    negative and looks as if it fitted the capacity.  The grid is refused, and
+    the engine works again with the particles back."""
+    rng = np.random.default_rng(1)
+    n = 300
+    x, y, z = rng.uniform(0, 1, (3, n))
+    o = np.ones(n)
+    arr = dict(x=x, y=y, z=z, u=0 * o, v=0 * o, w=0 * o, m=o, h=0.1 * o, rho=o, p=0 * o, cs=o)
+    eng = Engine([([arr], dict(dt=1e-9))], fluid_scheme(1), dim=3, precision=precision)
+    eng.density()
+    eng.check_status()
+    want = eng.get(0, "rho")
+    start = {c: eng.get(0, c) for c in "xyz"}
+    for c in "xyz":
+        eng.exchange_in(0, c, start[c] * (cells * eng.cell_size()))
+    eng.density()
+    assert eng.status() & nat.ST_GRID_OVERFLOW
+    for c in "xyz":
+        eng.exchange_in(0, c, start[c])
+    eng.rebin_now()
+    eng.clear_status()
+    eng.rebin_now()
+    eng.density()
+    eng.check_status()
+    assert torch.allclose(eng.get(0, "rho"), want, rtol=1e-6, atol=0)
