@@ -397,8 +397,8 @@ k_density(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask, in
         }
         if (active && !(lists_only && nbr)) {
             const double kf = Kern<KT>::template norm<DIM>();
-            const double ihk = 1.0 / hk;
-            const double fack = (DIM == 2 ? 1.0 / (hk * hk) : 1.0 / (hk * hk * hk)) * kf;
+            const double ihk = rcp_pair(hk);
+            const double fack = (DIM == 2 ? rcp_pair(hk * hk) : rcp_pair(hk * hk * hk)) * kf;
             struct Rec {
                 double x, y, z, m, h;
                 bool ok;

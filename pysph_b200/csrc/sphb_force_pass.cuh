@@ -440,8 +440,9 @@ k_force(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask,
         double dt_h = 1.0;
         // fac / h of the gradients, applied to the sums where one serves all
         // pairs: a product and a constant fewer in the loop, whose 96 registers
-        // spill (86k dam break 1,164 -> 1,146 us per 10 steps)
-        double scale = 1.0;
+        // spill (86k dam break 1,164 -> 1,146 us per 10 steps); w_scale: the
+        // same for XSPH's W, with eps
+        double scale = 1.0, w_scale = 1.0;
         if (active) {
             const int N = e.cfg.num_particles;
             const sphb_buffers &B = e.buf[cur];
@@ -466,9 +467,9 @@ k_force(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask,
             const double alpha = sc.alpha, beta = sc.beta, eta2 = sc.eta * sc.eta;
             const double kf = Kern<KT>::template norm<DIM>();
             const double alp_k = alpha * hk, bet2_k = 2.0 * beta * hk * hk;
-            const double ihk = 1.0 / hk;
-            const double fack = (DIM == 2 ? 1.0 / (hk * hk) : 1.0 / (hk * hk * hk)) * kf;
-            const double fihk = fack / hk;
+            const double ihk = rcp_pair(hk);
+            const double fack = (DIM == 2 ? rcp_pair(hk * hk) : rcp_pair(hk * hk * hk)) * kf;
+            const double fihk = fack * ihk;
             // with one h in the scene the symmetric set and the averaged
             // kernels are the plain ones
             const bool vh = sc.variable_h != 0, hks = sc.hks != 0;
@@ -480,7 +481,10 @@ k_force(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask,
             auto pass = [&](auto uniform) {
                 constexpr bool UH = decltype(uniform)::value;
                 if (UH) dt_h = hk;
-                if (UH) scale = fihk;
+                if (UH) {
+                    scale = fihk;
+                    w_scale = fack * sc.xsph_eps;
+                }
                 // KM as in the FP32C body: the mode known at compile time in
                 // the list loops, -1 in the cell search
                 auto make_load = [&](auto known) {
@@ -529,18 +533,24 @@ k_force(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask,
                         const double hab = UH ? hk : 0.5 * (hk + r.h);
                         double ir;
                         const double rr = dist_pair(r2, ir);
+                        // the quotient's residual matters to W, whose sum XSPH is,
+                        // not to the gradients' (accelerations 0.71 of the error
+                        // of divisions and square roots with it and without)
+                        auto q_of = [](double r, double h, double ih) {
+                            return CONT ? over_h(r, h, ih) : mul_pair(r, ih);
+                        };
                         // grad W / r (and W for XSPH) at h_ab, or with hks the
                         // means of the values at h_a and h_b (pressure_funcs.pyx:
                         // 371-381)
                         double gw, w = 0.0;
                         if (UH) {
-                            const double q = over_h(rr, hk, ihk);
+                            const double q = q_of(rr, hk, ihk);
                             gw = Kern<KT>::template gw_in<false>(q, ir, ihk, 1.0);
-                            if (CONT) w = Kern<KT>::template w_in<false>(q, fack);
+                            if (CONT) w = Kern<KT>::template w_in<false>(q, 1.0);
                         } else {
                             auto eval = [&](double hs, double ih, double fac, double fih,
                                             double &wh) {
-                                const double q = over_h(rr, hs, ih);
+                                const double q = q_of(rr, hs, ih);
                                 if (CONT) wh = Kern<KT>::template w_in<true>(q, fac);
                                 return Kern<KT>::template gw_in<true>(q, ir, ih, fih);
                             };
@@ -566,8 +576,10 @@ k_force(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask,
                             if (DIM == 3) d += vz * gz;
                             drho += rate_on ? d * r.m : 0.0;
                             // XSPHCorrection: m_b W_ab / rho_ab (v_b - v_a) eps
-                            const double temp =
-                                r.m * w * rcp_pair(0.5 * (r.rho + rhoa)) * sc.xsph_eps;
+                            // (eps with the normalisation, at the end, where one
+                            // serves all pairs)
+                            double temp = r.m * w * rcp_pair(0.5 * (r.rho + rhoa));
+                            if (!UH) temp *= sc.xsph_eps;
                             xs[0] -= xs_on ? temp * vx : 0.0;
                             xs[1] -= xs_on ? temp * vy : 0.0;
                             if (DIM == 3) xs[2] -= xs_on ? temp * vz : 0.0;
@@ -642,7 +654,11 @@ k_force(const __grid_constant__ sphb_engine e, int cur, uint32_t dest_mask,
         dtf *= dt_h;
 #pragma unroll
         for (int d = 0; d < DIM; ++d) acc[d] *= scale;
-        if (CONT) drho *= scale;
+        if (CONT) {
+            drho *= scale;
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) xs[d] *= w_scale;
+        }
     }
 
     force_finish<DIM, F32, CONT>(e, cur, k, s, a, active, lane, acc, dtf, drho, xs,
