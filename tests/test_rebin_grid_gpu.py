@@ -4,7 +4,6 @@ the cell table are reported."""
 import numpy as np
 import pytest
 import torch
-from cuda.bindings import driver
 
 from pysph_b200 import _native as nat
 from pysph_b200.engine import Engine, fluid_scheme
@@ -12,20 +11,20 @@ from pysph_b200.engine import Engine, fluid_scheme
 pytestmark = pytest.mark.gpu
 
 
-def _ok(res):
-    assert res[0] == driver.CUresult.CUDA_SUCCESS, res[0]
-    return res[1:]
-
-
 def _rebin_blocks(eng):
+    driver = pytest.importorskip("cuda.bindings.driver")
+
+    def ok(res):
+        assert res[0] == driver.CUresult.CUDA_SUCCESS, res[0]
+        return res[1:]
     eng.rebin_now()
     g = torch.cuda.CUDAGraph(keep_graph=True)
     with torch.cuda.graph(g):
         eng.call("sphb_bin", eng.cur, nat.BIN_IF_NEEDED)
     graph = driver.CUgraph(init_value=g.raw_cuda_graph())
-    _, n = _ok(driver.cuGraphGetNodes(graph, 0))
-    nodes, _ = _ok(driver.cuGraphGetNodes(graph, n))
-    return [_ok(driver.cuGraphKernelNodeGetParams(k))[0].gridDimX for k in nodes[:n]]
+    _, n = ok(driver.cuGraphGetNodes(graph, 0))
+    nodes, _ = ok(driver.cuGraphGetNodes(graph, n))
+    return [ok(driver.cuGraphKernelNodeGetParams(k))[0].gridDimX for k in nodes[:n]]
 
 
 def _engine(n, side, dim, **kw):
